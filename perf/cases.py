@@ -1,0 +1,365 @@
+"""What a user of this library has it do, as cases that can be timed and compared.
+
+A case is a dict of plain values; its "kind" says which public entry points the pass goes through:
+
+  linear   one planned GEMM (gemm_init once, gemm_exec per pass) on a weight that stays: a single quantised linear layer
+  wrapper  ABQGEMMWrapper.gemm, the class that replaces the one at the FasterTransformer call sites
+  engine   launch_pack on the activations, then the planned int32 GEMM on both operands' planes (the engine's own use)
+  torch    torch.ops.abq_b200.linear_half: the operator a torch program calls
+  decode   the linear layers of a stack of LLaMA blocks (TensorParallelBlockLinears) for one token step, captured in one
+           CUDA graph as a serving loop does; a pass is a replay
+  prefill  the same layers on a prompt, launched eagerly
+  prenorm  residual add -> RMSNorm -> per-token quantiser -> planes (one launch), then the GEMM that reads the planes
+  load     an fp16 weight quantised on the GPU when a model is loaded
+
+Sizes are those of LLaMA-7B (hidden 4096, FFN 11008) and LLaMA-2-13B (5120, 13824) and the ranges around them; weights and
+activations are synthetic, with the bit widths, scale groups and zero points of the library's configurations.
+"""
+from __future__ import annotations
+
+import importlib
+import importlib.util
+import math
+import sys
+from pathlib import Path
+
+import torch
+
+ROOT = Path(__file__).resolve().parent.parent
+
+
+def _package():
+    """The package directory's name has a hyphen: it is registered under an importable one."""
+    if "abq_llm_b200" not in sys.modules:
+        pkg = Path.cwd() / "abq-llm_b200"
+        if not pkg.is_dir():
+            pkg = ROOT / "abq-llm_b200"
+        spec = importlib.util.spec_from_file_location("abq_llm_b200", pkg / "__init__.py", submodule_search_locations=[str(pkg)])
+        mod = importlib.util.module_from_spec(spec)
+        sys.modules["abq_llm_b200"] = mod
+        spec.loader.exec_module(mod)
+    return sys.modules["abq_llm_b200"]
+
+
+abq = _package()
+B = importlib.import_module("abq_llm_b200.binding")
+TP = importlib.import_module("abq_llm_b200.tp_linear")
+importlib.import_module("abq_llm_b200.torch_ops")
+
+
+def listed():
+    return [
+        # the smallest call there is in earnest: one token through one projection, launch by launch
+        dict(name="linear_m1_w2a8_g128", kind="linear", M=1, N=4096, K=4096, w_bits=2, x_bits=8, group=128, zero=True, prepared=True),
+        # a few sequences decoding through the drop-in class: fp16 activations, planes as they were loaded, 8 tokens of an up projection
+        dict(name="wrapper_m8_w2a8", kind="wrapper", M=8, N=11008, K=4096, w_bits=2, x_bits=8),
+        # the engine's own check: a 128-row W4A4 problem, activations packed on the call, int32 out
+        dict(name="engine_m128_w4a4", kind="engine", M=128, N=4096, K=4096, w_bits=4, x_bits=4, signed=False),
+        # a torch program with a short prompt; widths and sizes off the beaten track (N odd, 23 blocks of 128 along K)
+        dict(name="torch_m77_w6a6", kind="torch", M=77, N=10007, K=2944, w_bits=6, x_bits=6, group=0, zero=True),
+        # token steps of the served models at the batch sizes of the end-to-end configurations
+        dict(name="decode_7b_w4a4_b1", kind="decode", M=1, hidden=4096, ffn=11008, blocks=4, w_bits=4, x_bits=4, group=0),
+        dict(name="decode_7b_w3a8_g128_b4", kind="decode", M=4, hidden=4096, ffn=11008, blocks=4, w_bits=3, x_bits=8, group=128),
+        dict(name="decode_13b_w2a8_g64_b16", kind="decode", M=16, hidden=5120, ffn=13824, blocks=3, w_bits=2, x_bits=8, group=64),
+        dict(name="decode_7b_w4a4_b32", kind="decode", M=32, hidden=4096, ffn=11008, blocks=4, w_bits=4, x_bits=4, group=0),
+        # one 512-token prompt
+        dict(name="prefill_7b_w4a4_512", kind="prefill", M=512, hidden=4096, ffn=11008, blocks=2, w_bits=4, x_bits=4, group=0),
+        # sixteen 1024-token prompts at once: the largest piece of work in the configurations
+        dict(name="prefill_13b_w2a8_g64_16k", kind="prefill", M=16384, hidden=5120, ffn=13824, blocks=1, w_bits=2, x_bits=8, group=64),
+        # norm, dynamic per-token quantiser and fused QKV of a 2048-token prompt, W8A8
+        dict(name="prenorm_m2048_w8a8", kind="prenorm", M=2048, N=12288, K=4096, w_bits=8, x_bits=8, prepared=True),
+        # one FFN weight on its way into the GPU: 4 bits, scale groups of 128
+        dict(name="load_w4_g128", kind="load", N=11008, K=4096, w_bits=4, group=128),
+    ]
+
+
+def _spread(rng, lo, hi, step=1):
+    """A multiple of ``step`` in lo..hi, even over the logarithm."""
+    v = math.exp(rng.uniform(math.log(lo), math.log(hi)))
+    return int(min(hi // step, max(-(-lo // step), round(v / step)))) * step
+
+
+def draw(rng):
+    kind = rng.choice(["linear", "linear", "wrapper", "engine", "torch", "decode", "decode", "decode", "prefill", "prefill", "prenorm", "load"])
+    if kind in ("decode", "prefill"):
+        hidden = _spread(rng, 2048, 5120, 128)
+        ffn = min(13824, int(hidden * rng.uniform(2.5, 3.5)) // 128 * 128)
+        w, x, g = rng.choice([(4, 4, 0), (4, 4, 0), (2, 8, 0), (8, 8, 0), (4, 8, 0), (2, 8, 64), (2, 8, 128), (3, 8, 128), (4, 8, 128)])
+        M = _spread(rng, 1, 64) if kind == "decode" else _spread(rng, 65, 8192)
+        return dict(kind=kind, M=M, hidden=hidden, ffn=ffn, blocks=rng.randint(2, 4) if kind == "decode" else 1, w_bits=w, x_bits=x, group=g)
+    N = _spread(rng, 1024, 14336) + rng.choice([0, 0, 1, 4])
+    K = _spread(rng, 1024, 13824, 128)
+    if kind == "linear":
+        M = _spread(rng, 1, 4096)
+        w, x, g = rng.choice([(2, 8, 128), (3, 8, 128), (4, 8, 128), (4, 4, 0), (8, 8, 0), (6, 6, 0), (5, 5, 0), (2, 4, 0), (2, 6, 0)])
+        return dict(kind=kind, M=M, N=N, K=K, w_bits=w, x_bits=x, group=g, zero=bool(g) or rng.random() < 0.5, prepared=rng.random() < 0.7)
+    if kind == "wrapper":
+        return dict(kind=kind, M=_spread(rng, 1, 512), N=(N + 7) // 8 * 8, K=K, w_bits=rng.choice([2, 2, 4, 8]), x_bits=8)
+    if kind == "engine":
+        w, x = rng.choice([(2, 2), (3, 3), (4, 4), (5, 5), (6, 6), (7, 7), (8, 8), (2, 4), (2, 6), (2, 8), (3, 8), (4, 8)])
+        return dict(kind=kind, M=_spread(rng, 1, 2048), N=N, K=K, w_bits=w, x_bits=x, signed=rng.random() < 0.5)
+    if kind == "torch":
+        w, x, g = rng.choice([(2, 8, 128), (4, 8, 128), (4, 4, 0), (8, 8, 0), (6, 6, 0), (3, 8, 0)])
+        return dict(kind=kind, M=_spread(rng, 1, 2048), N=N, K=K, w_bits=w, x_bits=x, group=g, zero=rng.random() < 0.7)
+    if kind == "prenorm":
+        w, x = rng.choice([(8, 8), (4, 4), (4, 8), (6, 6)])
+        return dict(kind=kind, M=_spread(rng, 1, 4096), N=N, K=K, w_bits=w, x_bits=x, prepared=rng.random() < 0.5)
+    return dict(kind="load", N=N, K=K, w_bits=rng.choice([2, 3, 4, 8]), group=rng.choice([0, 64, 128]))
+
+
+# ------------------------------------------------------------------------------------------------------------ inputs
+
+def _gen(seed):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    return g
+
+
+def _codes(gen, rows, K, bits, signed=False):
+    lo = -(1 << (bits - 1)) if signed else 0
+    return torch.randint(lo, lo + (1 << bits), (rows, K), dtype=torch.int32, device="cuda", generator=gen)
+
+
+def _planes(codes, bits):
+    rows, K = codes.shape
+    out = torch.empty((bits, rows, K // 32), dtype=torch.int32, device="cuda")
+    abq.pack_int32(codes, out, rows, K, bits)
+    return out
+
+
+def _weight_params(gen, N, K, bits, group, zero, gain=1.0):
+    """fp16 scales that keep the output of unit-variance activations near ``gain``, zero points beside the middle of the code range."""
+    shape = (N, K // group) if group else (N,)
+    step = gain * math.sqrt(12.0) / ((1 << bits) * math.sqrt(K))
+    scale = ((torch.rand(shape, device="cuda", generator=gen) + 0.5) * step).to(torch.float16)
+    mid = 1 << (bits - 1)
+    z = None
+    if zero:
+        z = (mid + torch.randint(-1, 1, shape, dtype=torch.int32, device="cuda", generator=gen)).clamp_(0, (1 << bits) - 1).to(torch.uint8)
+    return scale, z
+
+
+def _static_scale(x_bits):
+    """Static activation scale: codes reach their limits at six standard deviations."""
+    return (1 << (x_bits - 1)) / 6.0
+
+
+def _workspace(nbytes):
+    return torch.empty(max(256, nbytes), dtype=torch.uint8, device="cuda")
+
+
+def _planned(M, N, K, X, planes, out, *, w_bits, x_bits, x_signed, prepared, **kw):
+    """gemm_init as a program with fixed weights calls it, with the one-time preparation of the weights where asked for."""
+    work = _workspace(B.gemm_workspace_bytes(M, N, K, x_bits, w_bits))
+    args = dict(w_bits=w_bits, x_bits=x_bits, x_signed=x_signed, workspace=work, **kw)
+    flags = args.pop("flags", 0)
+    if not prepared:
+        p = B.make_params(M, N, K, X, planes, out, flags=flags, **args)
+        return abq.gemm_init(p), p
+    flags |= B.FLAG_WEIGHTS_PREPARED
+    nbytes = abq.gemm_prepared_weight_bytes(B.make_params(M, N, K, X, planes, out, flags=flags, **args)) if M <= 16 else 0
+    copy = torch.empty(nbytes, dtype=torch.uint8, device="cuda") if nbytes else None
+    p = B.make_params(M, N, K, X, planes, out, flags=flags, w_prepared=copy, **args)
+    state = abq.gemm_init(p)
+    abq.gemm_prepare_weights(state)
+    torch.cuda.synchronize()
+    return state, p
+
+
+def _prepare_linear(c, gen):
+    M, N, K, q, p = c["M"], c["N"], c["K"], c["w_bits"], c["x_bits"]
+    planes = _planes(_codes(gen, N, K, q), q)
+    scale, zero = _weight_params(gen, N, K, q, c["group"], c["zero"])
+    x = (torch.randn((M, K), device="cuda", generator=gen) * _static_scale(p)).round().clamp(-(1 << (p - 1)), (1 << (p - 1)) - 1).to(torch.int32)
+    xp = _planes(x, p)
+    x_scale = torch.rand((M,), device="cuda", generator=gen) * 0.1 + 0.05
+    out = torch.empty((M, N), dtype=torch.float16, device="cuda")
+    state, params = _planned(M, N, K, xp, planes, out, w_bits=q, x_bits=p, x_signed=True, w_signed=False, prepared=c["prepared"], out_dtype=B.OUT_FP16,
+                             scale_mode=B.SCALE_GROUP if c["group"] else B.SCALE_CHANNEL, group_size=c["group"], w_scale=scale, w_zero=zero, x_scale=x_scale)
+
+    def run():
+        abq.gemm_exec(state)
+        return out
+    return run, params
+
+
+def _prepare_wrapper(c, gen):
+    M, N, K, q, p = c["M"], c["N"], c["K"], c["w_bits"], c["x_bits"]
+    planes = _planes(_codes(gen, N, K, q, signed=True), q)
+    x = torch.randn((M, K), device="cuda", generator=gen).to(torch.float16)
+    scale = torch.full((1,), _static_scale(p), dtype=torch.float32, device="cuda")
+    # the product's scale, read by the class as fp16 from the start of the float
+    half_scale = torch.tensor([math.sqrt(12.0) / ((1 << q) * math.sqrt(K) * _static_scale(p)), 0.0], dtype=torch.float16, device="cuda")
+    scale_out = half_scale.view(torch.float32)
+    wrapper = abq.ABQGEMMWrapper(p, q, True)
+    work = _workspace(wrapper.workspace_bytes(M, N, K))
+    out = torch.empty((M, N), dtype=torch.float16, device="cuda")
+
+    def run():
+        wrapper.gemm(M, N, K, x, planes, None, out, scale, None, scale_out, False, work, work.numel())
+        return out
+    return run, (planes, work)
+
+
+def _prepare_engine(c, gen):
+    M, N, K, q, p, s = c["M"], c["N"], c["K"], c["w_bits"], c["x_bits"], c["signed"]
+    planes = _planes(_codes(gen, N, K, q, s), q)
+    x = _codes(gen, M, K, p, s)
+    xp = torch.empty((p, M, K // 32), dtype=torch.int32, device="cuda")
+    out = torch.empty((M, N), dtype=torch.int32, device="cuda")
+    state, params = _planned(M, N, K, xp, planes, out, w_bits=q, x_bits=p, x_signed=s, w_signed=s, prepared=False, out_dtype=B.OUT_INT32,
+                             scale_mode=B.SCALE_NONE)
+
+    def run():
+        abq.launch_pack(x, xp, M, K, p)
+        abq.gemm_exec(state)
+        return out
+    return run, params
+
+
+def _prepare_torch(c, gen):
+    M, N, K, q, p = c["M"], c["N"], c["K"], c["w_bits"], c["x_bits"]
+    planes = _planes(_codes(gen, N, K, q), q)
+    scale, zero = _weight_params(gen, N, K, q, c["group"], c["zero"])
+    x = torch.randn((M, K), device="cuda", generator=gen).to(torch.float16)
+    q_scale = torch.full((1,), _static_scale(p), dtype=torch.float32, device="cuda")
+    op = torch.ops.abq_b200.linear_half
+
+    def run():
+        return op(x, planes, scale, zero, q_scale, p, q, c["group"])
+    return run, None
+
+
+def _stack(c, gen):
+    q, group = c["w_bits"], c["group"]
+    backend = TP.AbqBackend(abq, torch, None, x_bits=c["x_bits"], x_scale=_static_scale(c["x_bits"]), max_tokens=c["M"])
+    # what the residual stream gains per block stays small, as it does in a trained network
+    gains = {"qkv": 1.0, "o": 0.3, "gate_up": 0.7, "down": 0.3}
+    blocks = []
+    for _ in range(c["blocks"]):
+        weights = []
+        for spec in TP.llama_block_specs(c["hidden"], c["ffn"]):
+            N, K = spec.out_features, spec.in_features
+            weights.append((_codes(gen, N, K, q), *_weight_params(gen, N, K, q, group, True, gains[spec.name])))
+        blocks.append(TP.TensorParallelBlockLinears(backend, c["hidden"], c["ffn"], 0, 1, weights, q, group))
+        del weights
+    x = torch.randn((c["M"], c["hidden"]), device="cuda", generator=gen).to(torch.float16)
+
+    def step():
+        h = x
+        for i, b in enumerate(blocks):  # a block writes its output where the next one reads its input
+            h = b.forward(h, blocks[i + 1].input_buffer(c["M"]) if i + 1 < len(blocks) else None)
+        return h
+    return step, blocks
+
+
+def _prepare_prefill(c, gen):
+    step, blocks = _stack(c, gen)
+    step()  # plans and buffers are made here
+    return step, blocks
+
+
+def _prepare_decode(c, gen):
+    step, blocks = _stack(c, gen)
+    step()
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        out = step()
+
+    def run():
+        graph.replay()
+        return out
+    return run, blocks
+
+
+def _prepare_prenorm(c, gen):
+    M, N, K, q, p = c["M"], c["N"], c["K"], c["w_bits"], c["x_bits"]
+    planes = _planes(_codes(gen, N, K, q), q)
+    scale, zero = _weight_params(gen, N, K, q, 0, True)
+    x = torch.randn((M, K), device="cuda", generator=gen).to(torch.float16)
+    residual = torch.randn((M, K), device="cuda", generator=gen).to(torch.float16)
+    gamma = (torch.rand((K,), device="cuda", generator=gen) + 0.5).to(torch.float16)
+    total = torch.empty_like(x)
+    row_scale = torch.empty((M,), dtype=torch.float32, device="cuda")
+    xp = torch.empty((p, M, K // 32), dtype=torch.int32, device="cuda")
+    out = torch.empty((M, N), dtype=torch.float16, device="cuda")
+    state, params = _planned(M, N, K, xp, planes, out, w_bits=q, x_bits=p, x_signed=True, w_signed=False, prepared=c["prepared"], out_dtype=B.OUT_FP16,
+                             scale_mode=B.SCALE_CHANNEL, w_scale=scale, w_zero=zero, x_scale=row_scale)
+
+    def run():
+        abq.rmsnorm_quantize_pack_half(x, gamma, 1e-6, M, K, p, 2, residual=residual, sum_out=total, row_scale_out=row_scale, planes=xp)
+        abq.gemm_exec(state)
+        return total, row_scale, out
+    return run, params
+
+
+def _prepare_load(c, gen):
+    N, K, q, g = c["N"], c["K"], c["w_bits"], c["group"]
+    w = (torch.randn((N, K), device="cuda", generator=gen) * 0.02).to(torch.float16)
+    planes = torch.empty((q, N, K // 32), dtype=torch.int32, device="cuda")
+    shape = (N, K // g) if g else (N,)
+    scale = torch.empty(shape, dtype=torch.float16, device="cuda")
+    zero = torch.empty(shape, dtype=torch.uint8, device="cuda")
+
+    def run():
+        abq.quantize_weights_half(w, planes, scale, zero, N, K, q, g)
+        return planes, scale, zero
+    return run, None
+
+
+_PREPARE = dict(linear=_prepare_linear, wrapper=_prepare_wrapper, engine=_prepare_engine, torch=_prepare_torch, decode=_prepare_decode,
+                prefill=_prepare_prefill, prenorm=_prepare_prenorm, load=_prepare_load)
+
+
+def prepare(case, seed):
+    """(the pass as a callable, what has to live as long as it)."""
+    return _PREPARE[case["kind"]](case, _gen(seed))
+
+
+def run(state):
+    return state[0]()
+
+
+# -------------------------------------------------------------------------------------------------- work and tolerance
+
+def _weight_bytes(N, K, q, group, zero=True):
+    return q * N * K // 8 + (2 + (1 if zero else 0)) * N * (K // group if group else 1)
+
+
+def work(case):
+    c, kind = case, case["kind"]
+    if kind in ("decode", "prefill"):
+        M, h, f = c["M"], c["hidden"], c["ffn"]
+        nbytes = flops = 0
+        for N, K in ((3 * h, h), (h, h), (2 * f, h), (h, f)):
+            nbytes += _weight_bytes(N, K, c["w_bits"], c["group"])
+            flops += 2 * M * N * K
+        # between the layers: every layer's fp16 input read and output written once
+        nbytes += 2 * M * ((h + 3 * h) + (h + h) + (h + 2 * f) + (f + h))
+        return {"bytes": c["blocks"] * nbytes, "flops": c["blocks"] * flops}
+    N, K, q = c["N"], c["K"], c["w_bits"]
+    if kind == "load":
+        return {"bytes": 2 * N * K + _weight_bytes(N, K, q, c["group"]), "flops": 0}
+    M, p = c["M"], c["x_bits"]
+    flops = 2 * M * N * K
+    if kind == "linear":
+        return {"bytes": _weight_bytes(N, K, q, c["group"], c["zero"]) + p * M * K // 8 + 4 * M + 2 * M * N, "flops": flops}
+    if kind == "wrapper":
+        return {"bytes": q * N * K // 8 + 2 * M * K + 2 * M * N, "flops": flops}
+    if kind == "engine":
+        return {"bytes": q * N * K // 8 + 4 * M * K + 4 * M * N, "flops": flops}
+    if kind == "torch":
+        return {"bytes": _weight_bytes(N, K, q, c["group"], c["zero"]) + 2 * M * K + 2 * M * N, "flops": flops}
+    return {"bytes": _weight_bytes(N, K, q, 0) + 3 * 2 * M * K + 2 * K + 2 * M * N, "flops": flops}  # prenorm
+
+
+def tolerance(case):
+    kind = case["kind"]
+    if kind in ("engine", "load"):
+        return "exact"  # integer sums; codes, scales and zero points follow one stated rule
+    # Against the same path with its sums in 64 bits: rel 2.1e-4 to 2.9e-4 (the rounding of the fp16 result) for single GEMMs,
+    # up to 1.7e-4 for the stacks.  max 8e-4 for one static quantiser; where a later quantiser can flip a code of another
+    # rounding upstream (stacks, dynamic per-token codes) 1.0e-2
+    return {"rel": 1e-3, "max": 4e-2 if kind in ("decode", "prefill", "prenorm") else 3e-3}
