@@ -166,13 +166,20 @@ def _planned(M, N, K, X, planes, out, *, w_bits, x_bits, x_signed, prepared, **k
     return state, p
 
 
-def _prepare_linear(c, gen):
+def _linear_inputs(c, gen):
     M, N, K, q, p = c["M"], c["N"], c["K"], c["w_bits"], c["x_bits"]
-    planes = _planes(_codes(gen, N, K, q), q)
+    codes = _codes(gen, N, K, q)
     scale, zero = _weight_params(gen, N, K, q, c["group"], c["zero"])
     x = (torch.randn((M, K), device="cuda", generator=gen) * _static_scale(p)).round().clamp(-(1 << (p - 1)), (1 << (p - 1)) - 1).to(torch.int32)
-    xp = _planes(x, p)
     x_scale = torch.rand((M,), device="cuda", generator=gen) * 0.1 + 0.05
+    return codes, scale, zero, x, x_scale
+
+
+def _prepare_linear(c, gen):
+    M, N, K, q, p = c["M"], c["N"], c["K"], c["w_bits"], c["x_bits"]
+    codes, scale, zero, x, x_scale = _linear_inputs(c, gen)
+    planes, xp = _planes(codes, q), _planes(x, p)
+    del codes, x
     out = torch.empty((M, N), dtype=torch.float16, device="cuda")
     state, params = _planned(M, N, K, xp, planes, out, w_bits=q, x_bits=p, x_signed=True, w_signed=False, prepared=c["prepared"], out_dtype=B.OUT_FP16,
                              scale_mode=B.SCALE_GROUP if c["group"] else B.SCALE_CHANNEL, group_size=c["group"], w_scale=scale, w_zero=zero, x_scale=x_scale)
@@ -183,13 +190,24 @@ def _prepare_linear(c, gen):
     return run, params
 
 
+def _half_inputs(c, gen, signed=False):
+    codes = _codes(gen, c["N"], c["K"], c["w_bits"], signed)
+    scale, zero = (None, None) if signed else _weight_params(gen, c["N"], c["K"], c["w_bits"], c["group"], c["zero"])
+    return codes, scale, zero, torch.randn((c["M"], c["K"]), device="cuda", generator=gen).to(torch.float16)
+
+
+def _product_scale(c):
+    return math.sqrt(12.0) / ((1 << c["w_bits"]) * math.sqrt(c["K"]) * _static_scale(c["x_bits"]))
+
+
 def _prepare_wrapper(c, gen):
     M, N, K, q, p = c["M"], c["N"], c["K"], c["w_bits"], c["x_bits"]
-    planes = _planes(_codes(gen, N, K, q, signed=True), q)
-    x = torch.randn((M, K), device="cuda", generator=gen).to(torch.float16)
+    codes, _, _, x = _half_inputs(c, gen, signed=True)
+    planes = _planes(codes, q)
+    del codes
     scale = torch.full((1,), _static_scale(p), dtype=torch.float32, device="cuda")
     # the product's scale, read by the class as fp16 from the start of the float
-    half_scale = torch.tensor([math.sqrt(12.0) / ((1 << q) * math.sqrt(K) * _static_scale(p)), 0.0], dtype=torch.float16, device="cuda")
+    half_scale = torch.tensor([_product_scale(c), 0.0], dtype=torch.float16, device="cuda")
     scale_out = half_scale.view(torch.float32)
     wrapper = abq.ABQGEMMWrapper(p, q, True)
     work = _workspace(wrapper.workspace_bytes(M, N, K))
@@ -201,10 +219,15 @@ def _prepare_wrapper(c, gen):
     return run, (planes, work)
 
 
+def _engine_inputs(c, gen):
+    return _codes(gen, c["N"], c["K"], c["w_bits"], c["signed"]), _codes(gen, c["M"], c["K"], c["x_bits"], c["signed"])
+
+
 def _prepare_engine(c, gen):
     M, N, K, q, p, s = c["M"], c["N"], c["K"], c["w_bits"], c["x_bits"], c["signed"]
-    planes = _planes(_codes(gen, N, K, q, s), q)
-    x = _codes(gen, M, K, p, s)
+    codes, x = _engine_inputs(c, gen)
+    planes = _planes(codes, q)
+    del codes
     xp = torch.empty((p, M, K // 32), dtype=torch.int32, device="cuda")
     out = torch.empty((M, N), dtype=torch.int32, device="cuda")
     state, params = _planned(M, N, K, xp, planes, out, w_bits=q, x_bits=p, x_signed=s, w_signed=s, prepared=False, out_dtype=B.OUT_INT32,
@@ -219,9 +242,9 @@ def _prepare_engine(c, gen):
 
 def _prepare_torch(c, gen):
     M, N, K, q, p = c["M"], c["N"], c["K"], c["w_bits"], c["x_bits"]
-    planes = _planes(_codes(gen, N, K, q), q)
-    scale, zero = _weight_params(gen, N, K, q, c["group"], c["zero"])
-    x = torch.randn((M, K), device="cuda", generator=gen).to(torch.float16)
+    codes, scale, zero, x = _half_inputs(c, gen)
+    planes = _planes(codes, q)
+    del codes
     q_scale = torch.full((1,), _static_scale(p), dtype=torch.float32, device="cuda")
     op = torch.ops.abq_b200.linear_half
 
@@ -230,17 +253,20 @@ def _prepare_torch(c, gen):
     return run, None
 
 
+def _block_weights(c, gen):
+    """(codes, scales, zero points) of QKV, attention output, gate/up and down."""
+    h, f = c["hidden"], c["ffn"]
+    # what the residual stream gains per block stays small, as it does in a trained network
+    return [(_codes(gen, N, K, c["w_bits"]), *_weight_params(gen, N, K, c["w_bits"], c["group"], True, gain))
+            for N, K, gain in ((3 * h, h, 1.0), (h, h, 0.3), (2 * f, h, 0.7), (h, f, 0.3))]
+
+
 def _stack(c, gen):
     q, group = c["w_bits"], c["group"]
     backend = TP.AbqBackend(abq, torch, None, x_bits=c["x_bits"], x_scale=_static_scale(c["x_bits"]), max_tokens=c["M"])
-    # what the residual stream gains per block stays small, as it does in a trained network
-    gains = {"qkv": 1.0, "o": 0.3, "gate_up": 0.7, "down": 0.3}
     blocks = []
     for _ in range(c["blocks"]):
-        weights = []
-        for spec in TP.llama_block_specs(c["hidden"], c["ffn"]):
-            N, K = spec.out_features, spec.in_features
-            weights.append((_codes(gen, N, K, q), *_weight_params(gen, N, K, q, group, True, gains[spec.name])))
+        weights = _block_weights(c, gen)
         blocks.append(TP.TensorParallelBlockLinears(backend, c["hidden"], c["ffn"], 0, 1, weights, q, group))
         del weights
     x = torch.randn((c["M"], c["hidden"]), device="cuda", generator=gen).to(torch.float16)
@@ -274,13 +300,20 @@ def _prepare_decode(c, gen):
     return run, blocks
 
 
-def _prepare_prenorm(c, gen):
-    M, N, K, q, p = c["M"], c["N"], c["K"], c["w_bits"], c["x_bits"]
-    planes = _planes(_codes(gen, N, K, q), q)
-    scale, zero = _weight_params(gen, N, K, q, 0, True)
+def _prenorm_inputs(c, gen):
+    M, K = c["M"], c["K"]
+    codes = _codes(gen, c["N"], K, c["w_bits"])
+    scale, zero = _weight_params(gen, c["N"], K, c["w_bits"], 0, True)
     x = torch.randn((M, K), device="cuda", generator=gen).to(torch.float16)
     residual = torch.randn((M, K), device="cuda", generator=gen).to(torch.float16)
-    gamma = (torch.rand((K,), device="cuda", generator=gen) + 0.5).to(torch.float16)
+    return codes, scale, zero, x, residual, (torch.rand((K,), device="cuda", generator=gen) + 0.5).to(torch.float16)
+
+
+def _prepare_prenorm(c, gen):
+    M, N, K, q, p = c["M"], c["N"], c["K"], c["w_bits"], c["x_bits"]
+    codes, scale, zero, x, residual, gamma = _prenorm_inputs(c, gen)
+    planes = _planes(codes, q)
+    del codes
     total = torch.empty_like(x)
     row_scale = torch.empty((M,), dtype=torch.float32, device="cuda")
     xp = torch.empty((p, M, K // 32), dtype=torch.int32, device="cuda")
@@ -320,6 +353,62 @@ def prepare(case, seed):
 
 def run(state):
     return state[0]()
+
+
+# ------------------------------------------------------------------------------------------------ the same in 64 bits
+
+def _static_codes(x, bits):
+    """The FasterTransformer quantiser: the fp16 product with the scale truncated to an integer, its low bits kept."""
+    q = (x.to(torch.float16) * torch.tensor(_static_scale(bits), dtype=torch.float32, device="cuda").to(torch.float16)).to(torch.int32)
+    half = 1 << (bits - 1)
+    return (((q + half) & (2 * half - 1)) - half).double()
+
+
+def _dequantised(codes, scale, zero, group):
+    w = codes.double()
+    N, K = w.shape
+    g = group or K
+    if zero is not None:
+        w = (w.view(N, K // g, g) - zero.double().view(N, K // g, 1)).view(N, K)
+    return (w.view(N, K // g, g) * scale.double().view(N, K // g, 1)).view(N, K)
+
+
+def exact(case, seed):
+    c, kind, gen = case, case["kind"], _gen(seed)
+    if kind == "linear":
+        codes, scale, zero, x, x_scale = _linear_inputs(c, gen)
+        return (x.double() @ _dequantised(codes, scale, zero, c["group"]).T) * x_scale.double().view(-1, 1)
+    if kind == "wrapper":
+        codes, _, _, x = _half_inputs(c, gen, signed=True)
+        return (_static_codes(x, c["x_bits"]) @ codes.double().T) * float(torch.tensor(_product_scale(c), dtype=torch.float16))
+    if kind == "engine":
+        codes, x = _engine_inputs(c, gen)
+        return (x.double() @ codes.double().T).to(torch.int32)  # below 2^53: exact
+    if kind == "torch":
+        codes, scale, zero, x = _half_inputs(c, gen)
+        return (_static_codes(x, c["x_bits"]) @ _dequantised(codes, scale, zero, c["group"]).T) / _static_scale(c["x_bits"])
+    if kind in ("decode", "prefill"):
+        weights = [_block_weights(c, gen) for _ in range(c["blocks"])]
+        y = torch.randn((c["M"], c["hidden"]), device="cuda", generator=gen).to(torch.float16).double()
+
+        def layer(v, w):
+            return (_static_codes(v, c["x_bits"]) @ _dequantised(*w, c["group"]).T) / _static_scale(c["x_bits"])
+        for qkv, o, gate_up, down in weights:
+            h = y + layer(layer(y, qkv)[:, :c["hidden"]], o)
+            gu = layer(h, gate_up)
+            act = torch.nn.functional.silu(gu[:, :c["ffn"]]) * gu[:, c["ffn"]:]
+            y = h + layer(act, down)
+        return y
+    if kind == "prenorm":
+        codes, scale, zero, x, residual, gamma = _prenorm_inputs(c, gen)
+        total = x.double() + residual.double()
+        y = total.to(torch.float16).double()
+        y = (y * torch.rsqrt((y * y).mean(1, keepdim=True) + 1e-6) * gamma.double()).to(torch.float16).double()
+        top = (1 << (c["x_bits"] - 1)) - 1
+        row_scale = y.abs().amax(1, keepdim=True) / top
+        q = (y / row_scale).round().clamp(-top - 1, top)
+        return total, row_scale.view(-1), (q @ _dequantised(codes, scale, zero, 0).T) * row_scale
+    return None  # load: codes, scales and zero points, compared bit for bit
 
 
 # -------------------------------------------------------------------------------------------------- work and tolerance
