@@ -781,15 +781,18 @@ __global__ void __launch_bounds__(MT == 4 ? 256 : kStreamMaxWarps * 32, 1) strea
             it_src[i] = live ? a.X + (size_t)m * (a.K >> 5) + (size_t)u0 * (UW / 32) + kwl : nullptr;
             const int ul = kwl / (UW / 32), part = kwl % (UW / 32);
             it_dst[i] = (uint32_t)(((size_t)ul * MR + m) * UW + part * 32) | (part == 0 ? 1u : 0u) | ((uint32_t)(m & 1) << 1);
+            // zero padding: by the thread that owns the place (there is no barrier between this and the records, and a padding
+            // store of another thread could land on top of one)
+            if (!live && idx < rec_items) {
+                uint4 *dst = reinterpret_cast<uint4 *>(rec_base + (it_dst[i] & ~3u));
+                dst[0] = dst[1] = make_uint4(0, 0, 0, 0);
+                if (part == 0)
+                    sums[ul * MR + m] = 0;
+            }
             if (live && (kwl & 31) == 0)
                 for (int b = 0; b < a.x_bits; ++b)
                     prefetch_l2(it_src[i] + b * a.x_plane_words);
         }
-        // zero padding: the whole record area (real items are overwritten after the wait)
-        for (int i = threadIdx.x; i < (int)((size_t)units_pad * MR * UW / 16); i += blockDim.x)
-            reinterpret_cast<uint4 *>(rec_base)[i] = make_uint4(0, 0, 0, 0);
-        for (int i = threadIdx.x; i < units_pad * MR; i += blockDim.x)
-            sums[i] = 0;
     } else {
         stream_build_records(a.X, a.x_plane_words, a.x_qscale, a.M, a.K, a.x_bits, a.x_signed, a.uw, rec_base, sums, u0, n_units, units_pad, MR, true);
     }
