@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) umma_kernel(const __grid_cons
     // Persistent CTA: tiles blockIdx.x, blockIdx.x + gridDim.x, ...; consecutive tiles share the weight (N) tile, so
     // the CTAs running at one time read few distinct weight tiles and all of the activations out of L2.
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int kc = 0; // k-blocks requested so far, over all tiles
             bool ok = true;
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) umma_kernel(const __grid_cons
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             int kc = 0, it = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) umma2_kernel(const __grid_con
     // Persistent CTA: tiles blockIdx.x, blockIdx.x + gridDim.x, ...; consecutive tiles share the weight (N) tile, so
     // the CTAs running at one time read few distinct weight tiles and all of the activations out of L2.
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int kc = 0; // k-blocks requested so far, over all tiles
             bool ok = true;
             for (int tile = pair; tile < total_tiles && ok; tile += pairs) {
@@ -467,7 +467,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) umma2_kernel(const __grid_con
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) { // the leader issues for the pair
+        if (rank == 0 && elect_one()) { // the leader issues for the pair
             int kc = 0, it = 0;
             bool ok = true;
             for (int tile = pair; tile < total_tiles && ok; tile += pairs, ++it) {
@@ -650,7 +650,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1) umma_group_kernel(const __gr
     pdl_wait_prior_grid();
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int kc = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1) umma_group_kernel(const __gr
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             int kc = 0, gc = 0; // K blocks and scale groups issued so far, over all tiles
             bool ok = true;
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
