@@ -83,10 +83,19 @@ cudaError_t umma_prepare_weights(const abq_gemm_state *st, cudaStream_t stream);
 cudaError_t umma_launch(const abq_gemm_state *st, cudaStream_t stream);
 size_t umma_workspace_bytes(int M, int N, int K);
 
+// ---- gemm_tc.cu (route ABQ_ROUTE_I8_UMMA: weights expanded from their planes inside the GEMM; per-group scales)
+// Plans on the route's workspace; scratch for split tiles may use [off_free, end).  expanded: weight codes in the workspace
+// (natural order, as the activation codes then are) instead of planes.  False: no launch for this problem.
+bool tc_plan(abq_gemm_state *st, int sms, size_t off_free, size_t end, bool expanded);
+bool tc_planned(const abq_gemm_state *st);  // tc_kernel, in either form
+bool tc_expanded(const abq_gemm_state *st); // ... over expanded codes
+cudaError_t tc_prepare_x(const abq_gemm_state *st, cudaStream_t stream); // activation codes into the workspace
+cudaError_t tc_launch(const abq_gemm_state *st, cudaStream_t stream);
+
 // ---- api.cu helpers
 // Encodes a tiled TMA descriptor through the driver entry point (no link-time libcuda dependency).
 // dims/strides innermost first; strides in bytes for dimensions 1..rank-1.
-enum TmapSwizzle { TMAP_SWIZZLE_NONE = 0, TMAP_SWIZZLE_64B = 2, TMAP_SWIZZLE_128B = 3 };
+enum TmapSwizzle { TMAP_SWIZZLE_NONE = 0, TMAP_SWIZZLE_32B = 1, TMAP_SWIZZLE_64B = 2, TMAP_SWIZZLE_128B = 3 };
 enum TmapDtype { TMAP_U8 = 0, TMAP_U32 = 1 };
 bool encode_tmap(void *out128, TmapDtype dtype, int rank, const void *base, const uint64_t *dims, const uint64_t *strides_bytes,
                  const uint32_t *box, TmapSwizzle swizzle);

@@ -60,6 +60,7 @@ bool encode_tmap(void *out128, TmapDtype dtype, int rank, const void *base, cons
                     const_cast<void *>(base), gdims, gstrides, gbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     swizzle == TMAP_SWIZZLE_128B  ? CU_TENSOR_MAP_SWIZZLE_128B
                     : swizzle == TMAP_SWIZZLE_64B ? CU_TENSOR_MAP_SWIZZLE_64B
+                    : swizzle == TMAP_SWIZZLE_32B ? CU_TENSOR_MAP_SWIZZLE_32B
                                                   : CU_TENSOR_MAP_SWIZZLE_NONE,
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
@@ -184,9 +185,9 @@ static abq_status plan_gemm(const abq_gemm_params *params, abq_gemm_state *state
     }
     int route = params->route;
     if (route == ABQ_ROUTE_AUTO) {
-        // up to 16 rows: one launch of the mma.sync route.  17..32 rows: two such launches still beat the tensor-core
-        // route, whose weight expansion alone costs more (measured on 12288x4096 and 4096x11008), unless the weight
-        // codes are already expanded.  Above: tcgen05.
+        // up to 16 rows: one launch of the mma.sync route.  17..32 rows: two such launches with scale groups (at 20 rows equal or a
+        // little faster than the tensor-core kernel) and for matrices of less than 4 Mi weights; otherwise (below) the
+        // tensor-core kernel over the planes, and always where the weight codes are already expanded.  Above: tcgen05.
         const int small = (params->flags & ABQ_FLAG_WEIGHTS_PREPARED) ? 16 : 32;
         route = params->M <= small ? ABQ_ROUTE_I8_MMA : ABQ_ROUTE_I8_UMMA;
     }
@@ -197,16 +198,28 @@ static abq_status plan_gemm(const abq_gemm_params *params, abq_gemm_state *state
         if (s == ABQ_ERR_UNSUPPORTED)
             route = ABQ_ROUTE_I8_MMA;
     }
+    // 17..32 rows: two launches of the mma.sync route against one of tc_kernel, W4A4, 32 rows: 12288 x 4096 27.2 -> 17.0 us,
+    // 4096 x 4096 17.8 -> 12.4, 22016 x 4096 38.2 -> 25.3, 4096 x 11008 35.3 -> 20.2.  A problem whose workspace does not hold
+    // that kernel's scratch keeps the two launches.
+    bool planes_kernel = false;
+    if (params->route == ABQ_ROUTE_AUTO && route == ABQ_ROUTE_I8_MMA && params->M > 16 && params->scale_mode != ABQ_SCALE_GROUP && !params->allreduce &&
+        (long long)params->N * params->K >= (4ll << 20)) {
+        planes_kernel = umma_plan(state) == ABQ_OK && tc_planned(state) && !tc_expanded(state);
+        if (planes_kernel)
+            route = ABQ_ROUTE_I8_UMMA;
+        else
+            std::memset(state->tmap, 0, sizeof(state->tmap));
+    }
     switch (route) {
     case ABQ_ROUTE_B1_MMA: s = b1_plan(state); break;
     case ABQ_ROUTE_I8_MMA: s = decode_plan(state, clear_counters); break;
-    case ABQ_ROUTE_I8_UMMA: s = umma_plan(state); break;
+    case ABQ_ROUTE_I8_UMMA: s = planes_kernel ? ABQ_OK : umma_plan(state); break;
     default: s = ABQ_ERR_INVALID_ARG;
     }
     if (s != ABQ_OK)
         return s;
-    if (params->residual && route != ABQ_ROUTE_I8_MMA)
-        return ABQ_ERR_UNSUPPORTED; // the residual add lives in the decode kernels' epilogues
+    if (params->residual && route != ABQ_ROUTE_I8_MMA && !planes_kernel)
+        return ABQ_ERR_UNSUPPORTED; // the residual add lives in the epilogues of the kernels for up to 32 rows
     state->route = route;
     state->p.allreduce = nullptr;
     if (state->ar.world > 0 && !(route == ABQ_ROUTE_I8_MMA && stream_planned(state) && state->cluster == 1))

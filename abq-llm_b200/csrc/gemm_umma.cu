@@ -17,12 +17,13 @@
 //               dequantisation, 16-byte stores; then the accumulator goes back to the MMA warp
 // Every wait is bounded (abq_common.cuh); on expiry the status word is set, the roles leave their loops, the
 // CTA still meets at the final barrier and TMEM is released.
-// Per-group scales: umma_group_kernel below (accumulator drained per scale group).
+// Per-group scales, and weights that are read as planes: tc_kernel (gemm_tc.cuh).
 #include <cuda.h>
 #include <cstring>
 
 #include "abq_common.cuh"
 #include "abq_kernels.h"
+#include "umma.cuh"
 
 namespace abq {
 
@@ -39,42 +40,10 @@ struct UmmaArgs {
     const uint8_t *w_zero;
     const float *x_scale;
     const int *xsum; // per-token code sums (only with per-channel zero points)
-    int kb_per_group;  // ABQ_SCALE_GROUP: 128-byte K blocks per scale group; 0: groups of 64 features, two per K block
-    int scale_groups;  // ABQ_SCALE_GROUP: scale groups per weight row
     int out_dtype, scale_mode;
     uint32_t idesc;
     int *status;
 };
-
-__device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t smem_addr)
-{
-    // K-major operand tile, 128-byte rows, SWIZZLE_128B: 8-row groups are 1024 B apart (stride byte offset);
-    // the leading byte offset is not used for swizzled K-major layouts (encoded as 1); descriptor version 1.
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr & 0x3ffff) >> 4);       // start address, 16-byte units, bits [0,14)
-    d |= (uint64_t)1 << 16;                            // leading byte offset (16 B units), bits [16,30)
-    d |= (uint64_t)(1024 >> 4) << 32;                  // stride byte offset (16 B units), bits [32,46)
-    d |= (uint64_t)1 << 46;                            // version (Blackwell), bits [46,48)
-    d |= (uint64_t)2 << 61;                            // layout type SWIZZLE_128B, bits [61,64)
-    return d;
-}
-
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile("{\n"
-                 ".reg .pred p;\n"
-                 "setp.ne.b32 p, %4, 0;\n"
-                 "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n"
-                 "}\n" ::"r"(tmem_d),
-                 "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-                 : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t *bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
 // 32 consecutive accumulator columns of this thread's TMEM lane
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, int (&v)[32])
@@ -155,20 +124,6 @@ __device__ __forceinline__ void store_chunk(const UmmaArgs &a, const int (&v)[32
                 dst[j] = __ushort_as_half((unsigned short)(h[j >> 1] >> ((j & 1) * 16)));
     }
 }
-
-// the same without the wait: several loads in flight, then one tmem_ld_wait()
-__device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, int (&v)[32])
-{
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-                   "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-                   "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-                   "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                 : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 template <int BN>
 __global__ void __launch_bounds__(kUmmaThreads, 1) umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
@@ -343,15 +298,6 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) umma_kernel(const __grid_cons
     }
 }
 
-// ---------------------------------------------------------------------------------------------------------------
-// ABQ_SCALE_GROUP on the tensor-core route: every scale group (kb_per_group K blocks) is multiplied into a fresh TMEM
-// accumulator, exactly, and the epilogue warps drain it while the next group is multiplied into the other one:
-//     facc[n] += scale[n][g] * acc_g[n]                                              (fp32, one row per thread)
-// The zero points are not seen here: the weight codes in the scratch are w - zero[n][g] (signed int8, exact for widths
-// up to 7 bits; see unpack_i8), so acc_g already is sum x * (w - z).  BN = 128 columns (128 fp32 partial sums per
-// thread); the scales of the tile, all groups, are staged once per tile in shared memory as fp32 [group][column].
-// MAGIC: |acc_g| < 2^22 (signed 8-bit activations, one K block per group): int -> float by the 1.5 * 2^23 trick, two
-// pipelined operations instead of a conversion instruction.  Same roles, barriers and bounded waits as umma_kernel.
 // cta_group::2 forms: issued by one thread of the even CTA of a pair
 __device__ __forceinline__ void umma2_i8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate)
 {
@@ -573,269 +519,6 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) umma2_kernel(const __grid_con
     }
 }
 
-// ---------------------------------------------------------------------------------------------------------------
-// ABQ_SCALE_GROUP on the tensor-core route: every scale group (kb_per_group K blocks) is multiplied into a fresh TMEM
-// accumulator, exactly, and the epilogue warps drain it while the next group is multiplied into the other one:
-//     facc[n] += scale[n][g] * acc_g[n]                                              (fp32, one row per thread)
-// The zero points are not seen here: the weight codes in the scratch are w - zero[n][g] (signed int8, exact for widths
-// up to 7 bits; see unpack_i8), so acc_g already is sum x * (w - z).  BN = 128 columns (128 fp32 partial sums per
-// thread); the scales of the tile, all groups, are staged once per tile in shared memory as fp32 [group][column].
-// MAGIC: |acc_g| < 2^22 (signed 8-bit activations, one K block per group): int -> float by the 1.5 * 2^23 trick, two
-// pipelined operations instead of a conversion instruction.  Same roles, barriers and bounded waits as umma_kernel.
-// facc[C .. C + 31] += scale[C .. C + 31] * float(v[0 .. 31]); the scales are the same for every lane (shared-memory broadcast)
-template <bool MAGIC, int C>
-__device__ __forceinline__ void scale_add(const int (&v)[32], const float *scales, float (&facc)[64])
-{
-#pragma unroll
-    for (int j = 0; j < 32; j += 4) {
-        const float4 sc = *reinterpret_cast<const float4 *>(scales + C + j);
-        const float s4[4] = { sc.x, sc.y, sc.z, sc.w };
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float fv = MAGIC ? __int_as_float(v[j + e] + 0x4b400000) - 12582912.0f : (float)v[j + e];
-            facc[C + j + e] = fmaf(s4[e], fv, facc[C + j + e]);
-        }
-    }
-}
-
-constexpr int kGroupBN = 128;
-constexpr int kGroupThreads = 320; // TMA warp, MMA warp, eight epilogue warps: two per TMEM lane quarter, 64 columns each
-
-template <bool MAGIC>
-__global__ void __launch_bounds__(kGroupThreads, 1) umma_group_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                                                                     const __grid_constant__ CUtensorMap tmap_b, const UmmaArgs a)
-{
-    extern __shared__ __align__(1024) uint8_t smem_raw[];
-    constexpr int BN = kGroupBN;
-    constexpr int kABytes = kUmmaBM * kUmmaBK, kBBytes = BN * kUmmaBK, kStageBytes = kABytes + kBBytes;
-    constexpr int kAccs = 4;              // accumulators in flight: the hand-over MMA -> epilogue -> MMA takes longer than two groups
-    constexpr int kTmemCols = kAccs * BN; // all 512 columns
-    // 1024-byte alignment as an offset from the array itself: a pointer rebuilt from an integer would lose its address space
-    // and every access behind it would compile to a generic load
-    uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    const int G = a.scale_groups;
-    float *s_scale = reinterpret_cast<float *>(smem + (size_t)a.stages * kStageBytes); // [G][BN]
-    uint64_t *bars = reinterpret_cast<uint64_t *>(s_scale + (size_t)G * BN);
-    uint64_t *full = bars, *empty = bars + 8, *acc_full = bars + 16, *acc_empty = bars + 20, *par_ready = bars + 24, *par_free = bars + 25;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 26);
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int k_blocks = a.K / kUmmaBK;
-    const int m_tiles = (a.M + kUmmaBM - 1) / kUmmaBM;
-    const int total_tiles = m_tiles * ((a.N + BN - 1) / BN);
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < a.stages; ++s) {
-            mbar_init(&full[s], 1);
-            mbar_init(&empty[s], 1);
-        }
-        for (int b = 0; b < kAccs; ++b) {
-            mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 8);
-        }
-        mbar_init(par_ready, 256); // the tile's scales are staged
-        mbar_init(par_free, 256);  // ... and no longer read (the next tile may overwrite them)
-        fence_mbar_init();
-        prefetch_tmap(&tmap_a);
-        prefetch_tmap(&tmap_b);
-    }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    tmem_fence_before();
-    __syncthreads();
-    tmem_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-    pdl_wait_prior_grid();
-
-    if (warp == 0) {
-        if (elect_one()) {
-            int kc = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-                const int m0 = (tile % m_tiles) * kUmmaBM, n0 = (tile / m_tiles) * BN;
-                for (int kb = 0; kb < k_blocks; ++kb, ++kc) {
-                    const int s = kc % a.stages;
-                    if (kc >= a.stages && !mbar_wait_bounded(&empty[s], ((kc / a.stages) - 1) & 1, a.status, STATUS_TIMEOUT_PIPE)) {
-                        ok = false;
-                        break;
-                    }
-                    uint8_t *sa = smem + (size_t)s * kStageBytes, *sb = sa + kABytes;
-                    mbar_arrive_expect_tx(&full[s], kStageBytes);
-                    tma_load_2d(sa, &tmap_a, kb * kUmmaBK, m0, &full[s]);
-                    tma_load_2d(sb, &tmap_b, kb * kUmmaBK, n0, &full[s]);
-                }
-            }
-        }
-        __syncwarp();
-    } else if (warp == 1) {
-        if (elect_one()) {
-            int kc = 0, gc = 0; // K blocks and scale groups issued so far, over all tiles
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-                if (a.kb_per_group == 0) {
-                    // scale groups of 64 features: a K block holds two groups; its first two MMAs start one accumulator, its
-                    // last two the next
-                    for (int kb = 0; kb < k_blocks && ok; ++kb, ++kc) {
-                        const int s = kc % a.stages;
-                        ok = mbar_wait_bounded(&full[s], (kc / a.stages) & 1, a.status, STATUS_TIMEOUT_TMA);
-                        if (!ok)
-                            break;
-                        tmem_fence_after();
-                        const uint32_t sa = smem_u32(smem + (size_t)s * kStageBytes), sb = sa + kABytes;
-                        const uint64_t da = make_smem_desc_sw128(sa), db = make_smem_desc_sw128(sb);
-                        for (int h = 0; h < 2 && ok; ++h, ++gc) {
-                            const int b = gc % kAccs;
-                            if (gc >= kAccs) {
-                                ok = mbar_wait_bounded(&acc_empty[b], ((gc / kAccs) - 1) & 1, a.status, STATUS_TIMEOUT_PIPE);
-                                if (!ok)
-                                    break;
-                                tmem_fence_after();
-                            }
-                            const uint32_t tmem_d = tmem_base + (uint32_t)(b * BN);
-#pragma unroll
-                            for (int k = 0; k < 2; ++k)
-                                umma_i8(tmem_d, da + (uint64_t)((2 * h + k) * 32 >> 4), db + (uint64_t)((2 * h + k) * 32 >> 4), a.idesc, k != 0);
-                            umma_commit(&acc_full[b]);
-                        }
-                        if (ok)
-                            umma_commit(&empty[s]);
-                    }
-                    continue;
-                }
-                for (int g = 0; g < G && ok; ++g, ++gc) {
-                    const int b = gc % kAccs;
-                    if (gc >= kAccs) { // the epilogue has drained this accumulator's previous group
-                        ok = mbar_wait_bounded(&acc_empty[b], ((gc / kAccs) - 1) & 1, a.status, STATUS_TIMEOUT_PIPE);
-                        if (!ok)
-                            break;
-                        tmem_fence_after();
-                    }
-                    const uint32_t tmem_d = tmem_base + (uint32_t)(b * BN);
-                    for (int kg = 0; kg < a.kb_per_group; ++kg, ++kc) {
-                        const int s = kc % a.stages;
-                        ok = mbar_wait_bounded(&full[s], (kc / a.stages) & 1, a.status, STATUS_TIMEOUT_TMA);
-                        if (!ok)
-                            break;
-                        tmem_fence_after();
-                        const uint32_t sa = smem_u32(smem + (size_t)s * kStageBytes), sb = sa + kABytes;
-                        const uint64_t da = make_smem_desc_sw128(sa), db = make_smem_desc_sw128(sb);
-#pragma unroll
-                        for (int k = 0; k < kUmmaBK / 32; ++k) // the first MMA of a group starts a fresh sum
-                            umma_i8(tmem_d, da + (uint64_t)(k * 32 >> 4), db + (uint64_t)(k * 32 >> 4), a.idesc, (kg | k) != 0);
-                        umma_commit(&empty[s]);
-                    }
-                    if (ok)
-                        umma_commit(&acc_full[b]);
-                }
-            }
-        }
-        __syncwarp();
-    } else {
-        const int quarter = warp & 3;          // the TMEM lanes a warp may read: 32 * (warp id % 4)
-        const int half = (warp - 2) >> 2;      // which 64 of the tile's 128 columns
-        const int et = threadIdx.x - 64;       // 0..255
-        constexpr int HN = BN / 2;
-        int gc = 0, it = 0;
-        bool ok = true;
-        for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
-            const int m0 = (tile % m_tiles) * kUmmaBM, n0 = (tile / m_tiles) * BN;
-            const int row = m0 + quarter * 32 + lane;
-            // ---- stage the scales of weight row n0 + et, all groups, as [group][column]
-            if (it > 0) {
-                ok = mbar_wait_bounded(par_free, (it - 1) & 1, a.status, STATUS_TIMEOUT_PIPE);
-                if (!ok)
-                    break;
-            }
-            {
-                const int col = et & (BN - 1), n = n0 + col;
-                const __half *src = a.w_scale + (size_t)(n < a.N ? n : 0) * G;
-                for (int g = et >> 7; g < G; g += 2) // two threads per weight row, alternate groups
-                    s_scale[(size_t)g * BN + col] = n < a.N ? __half2float(src[g]) : 0.f;
-            }
-            mbar_arrive(par_ready);
-            ok = mbar_wait_bounded(par_ready, it & 1, a.status, STATUS_TIMEOUT_PIPE);
-            if (!ok)
-                break;
-            float xs = 1.f;
-            if (row < a.M && a.x_scale)
-                xs = a.x_scale[row];
-            float facc[HN];
-#pragma unroll
-            for (int c = 0; c < HN; ++c)
-                facc[c] = 0.f;
-            // Pipelined over 32-column chunks: while chunk i is scaled and added, the tcgen05.ld of chunk i + 1 (the second
-            // half of this group, or the first half of the next group) is already in flight; an accumulator goes back
-            // to the MMA warp as soon as its second half sits in registers.
-            int va[32], vb[32];
-            const uint32_t tlane = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * HN);
-            {
-                const int b = gc % kAccs;
-                ok = mbar_wait_bounded(&acc_full[b], (gc / kAccs) & 1, a.status, STATUS_TIMEOUT_MMA);
-                if (!ok)
-                    break;
-                tmem_fence_after();
-                tmem_ld32_nowait(tlane + (uint32_t)(b * BN), va);
-            }
-            for (int g = 0; g < G; ++g) {
-                const int b = gc % kAccs;
-                const float *sg = s_scale + (size_t)g * BN + half * HN;
-                tmem_ld_wait();                                         // first half of group g is in va
-                tmem_ld32_nowait(tlane + (uint32_t)(b * BN + 32), vb);  // second half on its way
-                scale_add<MAGIC, 0>(va, sg, facc);
-                tmem_ld_wait();                                         // second half in vb: the accumulator is free
-                tmem_fence_before();
-                __syncwarp();
-                if (lane == 0)
-                    mbar_arrive(&acc_empty[b]);
-                ++gc;
-                if (g + 1 < G) {
-                    const int nb = gc % kAccs;
-                    ok = mbar_wait_bounded(&acc_full[nb], (gc / kAccs) & 1, a.status, STATUS_TIMEOUT_MMA);
-                    if (!ok)
-                        break;
-                    tmem_fence_after();
-                    tmem_ld32_nowait(tlane + (uint32_t)(nb * BN), va);  // first half of group g + 1 on its way
-                }
-                scale_add<MAGIC, 32>(vb, sg, facc);
-            }
-            mbar_arrive(par_free); // this thread reads the staged parameters no more
-            if (!ok)
-                break;
-            if (row < a.M) {
-                const int nb = n0 + half * HN;
-                __half *dst = reinterpret_cast<__half *>(a.D) + (size_t)row * a.N + nb;
-                const bool vec = nb + HN <= a.N && (a.N & 7) == 0;
-#pragma unroll
-                for (int c = 0; c < HN; c += 8) {
-                    uint32_t h[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const __half2 t = __floats2half2_rn(facc[c + 2 * e] * xs, facc[c + 2 * e + 1] * xs);
-                        h[e] = *reinterpret_cast<const uint32_t *>(&t);
-                    }
-                    if (vec) {
-                        *reinterpret_cast<uint4 *>(dst + c) = make_uint4(h[0], h[1], h[2], h[3]);
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            if (nb + c + e < a.N)
-                                dst[c + e] = __ushort_as_half((unsigned short)(h[e >> 1] >> ((e & 1) * 16)));
-                    }
-                }
-            }
-        }
-    }
-
-    tmem_fence_before();
-    __syncthreads();
-    if (warp == 1) {
-        tmem_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
-    }
-}
-
 // per-token sum of the int8 / uint8 activation codes (needed only with weight zero points)
 __global__ void __launch_bounds__(256) rowsum_kernel(const uint8_t *__restrict__ x, int *__restrict__ out, int M, int K, int is_signed)
 {
@@ -892,14 +575,14 @@ abq_status umma_plan(abq_gemm_state *st)
     const bool grouped = p.scale_mode == ABQ_SCALE_GROUP;
     const int scale_groups = grouped ? p.K / p.group_size : 0;
     if (grouped) {
-        // drained per scale group (umma_group_kernel): groups of whole K blocks; zero points are folded into the int8
+        // drained per scale group (tc_kernel): groups of whole K blocks; zero points are folded into the int8
         // weight codes, which needs w - z to fit: unsigned weights of at most 7 bits
         if ((p.group_size % kUmmaBK != 0 && p.group_size != kUmmaBK / 2) || p.out_dtype != ABQ_OUT_FP16)
-            return ABQ_ERR_UNSUPPORTED; // (groups of 64: two per K block, see the MMA warp of umma_group_kernel)
+            return ABQ_ERR_UNSUPPORTED; // (groups of 64: two per K block)
         if (p.w_zero && (p.w_signed || p.w_bits > 7))
             return ABQ_ERR_UNSUPPORTED;
-        if ((size_t)scale_groups * kGroupBN * 4 + 3 * (size_t)(kUmmaBM + kGroupBN) * kUmmaBK > 216 * 1024)
-            return ABQ_ERR_UNSUPPORTED; // the tile's scales would not fit beside three stages
+        if ((size_t)scale_groups * 512 > 120 * 1024)
+            return ABQ_ERR_UNSUPPORTED; // (as many groups per row as this route has always taken)
     }
     size_t off_w, off_sum, total;
     umma_layout(p.M, p.N, p.K, &off_w, &off_sum, &total);
@@ -913,6 +596,19 @@ abq_status umma_plan(abq_gemm_state *st)
         if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0)
             sms = v;
     }
+    // Weights straight from their planes (tc_kernel) while the token tiles of a weight tile are few: expanding a tile once per
+    // token tile inside the GEMM is then cheaper than writing and re-reading the whole expanded matrix.  W4A4, whole call, this
+    // route before and now: 12288 x 4096 33.5 -> 18.9 us at 64 tokens, 35.6 -> 24.5 at 128, 40.3 -> 33.3 at 256, equal at 512.
+    // Rows of D that are not multiples of 16 bytes cost umma_kernel a store per value, tc_kernel nothing: 10007 x 2944 44.8 -> 20.5
+    // us at 128 tokens, 103 -> 48 at 512, 156 -> 113 at 1024.  With scale groups (2 bits, groups of 64) 12288 x 4096 55.1 -> 33.2 at 64
+    // tokens, equal at 128.  Weights that were expanded beforehand keep the kernels that read codes.
+    const bool ragged = p.N % (p.out_dtype == ABQ_OUT_INT32 ? 4 : 8) != 0;
+    const int planes_rows = env_int("ABQ_TC_ROWS", grouped ? 128 : (ragged ? 4096 : 256));
+    const bool pairs_asked = env_int("ABQ_UMMA_PAIRS", 0) != 0;
+    if (!(p.flags & ABQ_FLAG_WEIGHTS_PREPARED) && !pairs_asked && p.M <= planes_rows && tc_plan(st, sms, off_w, off_sum, false))
+        return ABQ_OK;
+    if (grouped)
+        return tc_plan(st, sms, total, total, true) ? ABQ_OK : ABQ_ERR_UNSUPPORTED;
     // N tile: the persistent CTAs run ceil(tiles / SMs) tiles each.  Narrower tiles balance better, but measured per
     // output column they cost almost twice as much (operand fetch per operation doubles), so they only win on small grids
     const int m_tiles = (p.M + kUmmaBM - 1) / kUmmaBM;
@@ -931,14 +627,12 @@ abq_status umma_plan(abq_gemm_state *st)
     BN = env_int("ABQ_UMMA_BN", BN);
     if (BN != 64 && BN != 128 && BN != 256)
         return ABQ_ERR_INVALID_ARG;
-    if (grouped)
-        BN = kGroupBN;
     // CTA pairs (256 x 256 tiles, umma2_kernel): a third less operand traffic per SM and six stages.  Measured equal to the
     // single-CTA kernel on the LLaMA shapes (that one already runs at the rate its rounds of tiles allow), so it is
     // opt-in: ABQ_UMMA_PAIRS=1
-    const bool paired = !grouped && BN == 256 && p.M > kUmmaBM && env_int("ABQ_UMMA_PAIRS", 0) != 0;
+    const bool paired = BN == 256 && p.M > kUmmaBM && pairs_asked;
     const int stage_bytes = paired ? (kUmmaBM + kPairBN / 2) * kUmmaBK : (kUmmaBM + BN) * kUmmaBK;
-    const size_t param_bytes = grouped ? (size_t)scale_groups * kGroupBN * 4 : (size_t)4 * BN * 4;
+    const size_t param_bytes = (size_t)4 * BN * 4;
     int stages = (int)((216 * 1024 - param_bytes) / stage_bytes);
     stages = stages > 8 ? 8 : stages;
     const int k_blocks = p.K / kUmmaBK;
@@ -963,13 +657,13 @@ abq_status umma_plan(abq_gemm_state *st)
         st->grid[0] = (unsigned)(tiles < sms ? tiles : sms); // persistent: a CTA per SM, tiles dealt round-robin
     st->grid[1] = 1;
     st->grid[2] = 1;
-    st->block[0] = grouped ? kGroupThreads : kUmmaThreads;
+    st->block[0] = kUmmaThreads;
     st->block[1] = st->block[2] = 1;
     st->cluster = paired ? 2 : 1;
     st->shared_mem_size = 1024 + (size_t)stages * stage_bytes + param_bytes + 256;
     st->tile[0] = BN;
     st->tile[1] = stages;
-    st->tile[2] = grouped ? 1 : (paired ? 2 : 0);
+    st->tile[2] = paired ? 2 : 0;
     return ABQ_OK;
 }
 
@@ -1005,13 +699,6 @@ static cudaError_t launch_kernel(Kernel kern, SmemOptIn *opted, const abq_gemm_s
         cfg.numAttrs = 2;
     }
     return cudaLaunchKernelEx(&cfg, kern, ta, tb, args);
-}
-
-template <bool MAGIC>
-static cudaError_t launch_group(const abq_gemm_state *st, const UmmaArgs &args, cudaStream_t stream)
-{
-    static thread_local SmemOptIn opted;
-    return launch_kernel(umma_group_kernel<MAGIC>, &opted, st, args, stream);
 }
 
 static cudaError_t launch_pair(const abq_gemm_state *st, const UmmaArgs &args, cudaStream_t stream)
@@ -1056,7 +743,10 @@ cudaError_t umma_launch(const abq_gemm_state *st, cudaStream_t stream)
     umma_layout(p.M, p.N, p.K, &off_w, &off_sum, &total);
     uint8_t *ws = reinterpret_cast<uint8_t *>(p.workspace);
     cudaError_t e;
-    if (p.flags & ABQ_FLAG_X_HALF) { // fp16 activations: quantise straight to codes; weights as usual
+    const bool tc = tc_planned(st);
+    if (tc && !tc_expanded(st))
+        e = tc_prepare_x(st, stream);
+    else if (p.flags & ABQ_FLAG_X_HALF) { // fp16 activations: quantise straight to codes; weights as usual
         e = cudaSuccess;
         if (!(p.flags & ABQ_FLAG_WEIGHTS_PREPARED))
             e = unpack_i8(reinterpret_cast<const uint32_t *>(p.W), ws + off_w, p.N, p.K, p.w_bits, p.w_signed, stream, folded_zero(p),
@@ -1070,6 +760,8 @@ cudaError_t umma_launch(const abq_gemm_state *st, cudaStream_t stream)
                            ws + off_w, p.N, p.w_bits, p.w_signed, p.K, stream, folded_zero(p), folded_group(p));
     if (e != cudaSuccess)
         return e;
+    if (tc)
+        return tc_launch(st, stream);
     UmmaArgs a;
     a.xsum = nullptr;
     if (p.scale_mode == ABQ_SCALE_CHANNEL && p.w_zero && !folded_zero(p)) {
@@ -1097,16 +789,9 @@ cudaError_t umma_launch(const abq_gemm_state *st, cudaStream_t stream)
     a.idesc = (2u << 4) | ((p.x_signed ? 1u : 0u) << 7) | ((b_signed ? 1u : 0u) << 10) | ((uint32_t)(BN >> 3) << 17) |
               ((uint32_t)(kUmmaBM >> 4) << 24);
     a.status = p.status_word;
-    a.kb_per_group = p.scale_mode == ABQ_SCALE_GROUP ? p.group_size / kUmmaBK : 0;
-    a.scale_groups = p.scale_mode == ABQ_SCALE_GROUP ? p.K / p.group_size : 0;
     if (st->tile[2] == 2) { // CTA pairs: one instruction covers 256 rows
         a.idesc = (a.idesc & ~(0x1fu << 24)) | ((uint32_t)(2 * kUmmaBM >> 4) << 24);
         return launch_pair(st, a, stream);
-    }
-    if (st->tile[2]) {
-        // |acc of a group| < 2^22 with signed activations (|x| <= 128), |w - z| <= 255 and one K block per group
-        const bool magic = p.x_signed && a.kb_per_group <= 1;
-        return magic ? launch_group<true>(st, a, stream) : launch_group<false>(st, a, stream);
     }
     switch (BN) {
     case 64: return launch_bn<64>(st, a, stream);

@@ -205,7 +205,11 @@ class AbqLinear:
             probe = B.make_params(M, self.out_features, self.in_features, x_view, self.planes, out, flags=flags, **kw)
             nbytes = self.abq.gemm_prepared_weight_bytes(probe) if M <= 32 else 0
             st = None
-            if nbytes:
+            if 16 < M <= 32 and fused is None:  # one launch of the tensor-core kernel instead of two on the prepared weights, where the planner says so
+                st = self.abq.gemm_init(probe)
+                if st.route != self.abq.ROUTE_I8_UMMA:
+                    st = None
+            if nbytes and st is None:
                 if self.prepared is None:
                     self.prepared = self.torch.empty(nbytes, dtype=self.torch.uint8, device="cuda")
                 try:
