@@ -150,7 +150,7 @@ typedef struct abq_gemm_params {
     void *w_prepared;           /* ABQ_FLAG_WEIGHTS_PREPARED on route I8_MMA: the re-ordered weights, 16-byte aligned */
     const abq_fused_allreduce *allreduce; /* optional (host pointer, copied by abq_gemm_init): sum D over the ranks inside the
                                              GEMM; plans that cannot do it answer ABQ_ERR_UNSUPPORTED */
-    const void *residual;   /* optional fp16 [M][N] (fp16 output, route I8_MMA; other plans answer ABQ_ERR_UNSUPPORTED):
+    const void *residual;   /* optional fp16 [M][N] (fp16 output; route I8_MMA, or AUTO up to 32 rows; other plans answer ABQ_ERR_UNSUPPORTED):
                                D = half(result) + residual, the fp16 add a separate residual kernel would do after the GEMM
                                (after the sum over the ranks when `allreduce` is set); may alias neither X nor D */
 } abq_gemm_params;
