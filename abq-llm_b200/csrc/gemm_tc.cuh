@@ -721,11 +721,17 @@ __global__ void __launch_bounds__((4 + E + EW) * 32, 1)
                 const bool g64 = a.group_size == 64;
                 const uint64_t minus2 = pack2(__float_as_uint(-a.magic_f), __float_as_uint(-a.magic_f));
                 const __half *srow = a.w_scale + (size_t)(row.live ? row.n : 0) * a.scale_groups;
+                // groups of 64: an even number of them per row, so a K block's two lie in one word -- where the array starts on one
+                // (a caller's view into a larger fp16 buffer need not)
+                const bool scale_words = (reinterpret_cast<uintptr_t>(a.w_scale) & 3) == 0;
                 const int units = g64 ? sg.k1 - sg.k0 : (sg.k1 - sg.k0 + 1) >> 1;
                 // the scale group of accumulator h of unit u (groups of at least a K block)
                 auto group_of = [&](int u, int h) { return tc_group_of(a, min(sg.k0 + 2 * u + h, sg.k1 - 1)); };
-                auto fetch = [&](int u) -> __half2 { // (groups of 64: an even number of them per row, both in one word)
-                    return g64 ? *reinterpret_cast<const __half2 *>(srow + 2 * (sg.k0 + u)) : __halves2half2(ld_half(srow + group_of(u, 0)), ld_half(srow + group_of(u, 1)));
+                auto fetch = [&](int u) -> __half2 {
+                    if (g64 && scale_words)
+                        return *reinterpret_cast<const __half2 *>(srow + 2 * (sg.k0 + u));
+                    const int g0 = g64 ? 2 * (sg.k0 + u) : group_of(u, 0), g1 = g64 ? g0 + 1 : group_of(u, 1);
+                    return __halves2half2(ld_half(srow + g0), ld_half(srow + g1));
                 };
                 __half2 scales = fetch(0);
                 for (int u = 0; u < units; ++u, ++unit) {

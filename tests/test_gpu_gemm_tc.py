@@ -66,3 +66,27 @@ def test_channel_zero_points(abq, oracle, cuda, q, w_signed):
                        route=abq.ROUTE_I8_UMMA, out_fp16=True, scale_mode=abq.SCALE_CHANNEL, w_scale=dev(scale), w_zero=dev(zero), x_scale=dev(xs))
     acc = oracle.gemm_values_blas(x, w).astype(np.float64) - zero.astype(np.float64)[None, :] * x.sum(axis=1, dtype=np.int64)[:, None]
     check_close(got, acc * scale.astype(np.float64)[None, :] * xs.astype(np.float64)[:, None])
+
+
+@pytest.mark.parametrize("M", [24, 100, 200])
+def test_scales_of_groups_of_64_off_a_word(abq, oracle, cuda, M):
+    """fp16 scales that start two bytes off a 32-bit word (a view into a larger buffer) give the bits that an aligned copy gives,
+    over planes (24, 100 rows) and over expanded codes (200)."""
+    N, K, q, group = 200, 1152, 3, 64
+    rng = np.random.default_rng(M)
+    x, w = rand_codes(rng, M, K, 8, True), rand_codes(rng, N, K, q, False)
+    G = K // group
+    flat = dev(rng.uniform(0.001, 0.02, size=N * G + 2).astype(np.float16))
+    off = flat[1:1 + N * G].view(N, G)
+    assert off.data_ptr() % 4 == 2 and off.is_contiguous()
+    aligned = off.clone()
+    zero = rng.integers(0, 1 << q, size=(N, G)).astype(np.uint8)
+    tok = rng.uniform(0.001, 0.01, size=M).astype(np.float32)
+    got = []
+    for scale in (aligned, off):
+        d, st = run_gemm(abq, planes_dev(oracle, x, 8), planes_dev(oracle, w, q), M, N, K, x_bits=8, w_bits=q, x_signed=True, w_signed=False,
+                         out_fp16=True, scale_mode=abq.SCALE_GROUP, group_size=group, w_scale=scale, w_zero=dev(zero), x_scale=dev(tok),
+                         route=abq.ROUTE_I8_UMMA)
+        got.append(d)
+    check_close(got[0], oracle.dequant_gemm(x, w, aligned.cpu().numpy(), zero.astype(np.int32), tok, group))
+    assert np.array_equal(got[0].view(np.uint16), got[1].view(np.uint16))
