@@ -224,6 +224,7 @@ def gemm(params: GemmParams, stream=None) -> None:
 
 
 STATIC_SCRATCH_BYTES = 16 << 20
+WORKSPACE_COUNTER_BYTES = 256 << 10  # the part of gemm_workspace_bytes() that only plans sharing a workspace need
 
 
 def gemm_static_scratch(params: GemmParams, stream=None) -> None:

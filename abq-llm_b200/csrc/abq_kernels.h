@@ -61,8 +61,10 @@ abq_status decode_plan(abq_gemm_state *st, bool clear_counters);
 cudaError_t decode_clear_counters(const abq_gemm_state *st, cudaStream_t stream);
 cudaError_t decode_launch(const abq_gemm_state *st, cudaStream_t stream);
 size_t decode_workspace_bytes(int M, int N, int K);
-// split-K scratch shared by both decode kernels: [tile counters][partial slots for kDecodeMaxSlices slices]
-void decode_workspace_layout(int M, int N, size_t *off_partials, size_t *total);
+// split-K scratch shared by both decode kernels: [tile counters][partial slots for kDecodeMaxSlices slices].  The counters have to outlive
+// the launches of every plan that shares the workspace: no plan puts anything else into its first ABQ_WORKSPACE_COUNTER_BYTES, where the
+// workspace has room for that
+void decode_workspace_layout(int M, int N, size_t bytes, size_t *off_partials, size_t *total); // in a workspace of `bytes`
 
 // ---- gemm_stream.cu (route ABQ_ROUTE_I8_MMA over prepared weights, ABQ_FLAG_WEIGHTS_PREPARED + w_prepared)
 bool stream_supported(const abq_gemm_params &p);
@@ -81,18 +83,25 @@ cudaError_t b1_launch(const abq_gemm_state *st, cudaStream_t stream);
 abq_status umma_plan(abq_gemm_state *st);
 cudaError_t umma_prepare_weights(const abq_gemm_state *st, cudaStream_t stream);
 cudaError_t umma_launch(const abq_gemm_state *st, cudaStream_t stream);
-size_t umma_workspace_bytes(int M, int N, int K);
+size_t umma_workspace_bytes(int M, int N, int K); // without the room for the decode plans' counters
+// Workspace of a plan (byte offsets): activation codes M x K, weight codes N x K, token sums M.  The first ABQ_WORKSPACE_COUNTER_BYTES are
+// left to the decode plans' counters where there is room for that (base = 0: there is not).
+struct UmmaLayout {
+    size_t base, x, w, sum, end;
+};
+UmmaLayout umma_layout(const abq_gemm_params &p);
 
 // ---- gemm_tc.cu (route ABQ_ROUTE_I8_UMMA: weights expanded from their planes inside the GEMM; per-group scales)
-// Plans on the route's workspace; scratch for split tiles may use [off_free, end).  expanded: weight codes in the workspace
-// (natural order, as the activation codes then are) instead of planes.  False: no launch for this problem.
-bool tc_plan(abq_gemm_state *st, int sms, size_t off_free, size_t end, bool expanded);
+// Plans on the route's workspace.  expanded: weight codes in the workspace (natural order, as the activation codes then are) instead of
+// planes; otherwise scratch for split tiles may use the weight codes' place.  False: no launch for this problem.
+bool tc_plan(abq_gemm_state *st, int sms, const UmmaLayout &L, bool expanded);
 bool tc_planned(const abq_gemm_state *st);  // tc_kernel, in either form
 bool tc_expanded(const abq_gemm_state *st); // ... over expanded codes
 cudaError_t tc_prepare_x(const abq_gemm_state *st, cudaStream_t stream); // activation codes into the workspace
 cudaError_t tc_launch(const abq_gemm_state *st, cudaStream_t stream);
 
 // ---- api.cu helpers
+size_t gemm_scratch_bytes(int M, int N, int K, int route); // abq_gemm_workspace_bytes() without ABQ_WORKSPACE_COUNTER_BYTES
 // Encodes a tiled TMA descriptor through the driver entry point (no link-time libcuda dependency).
 // dims/strides innermost first; strides in bytes for dimensions 1..rank-1.
 enum TmapSwizzle { TMAP_SWIZZLE_NONE = 0, TMAP_SWIZZLE_32B = 1, TMAP_SWIZZLE_64B = 2, TMAP_SWIZZLE_128B = 3 };

@@ -146,6 +146,14 @@ size_t abq_gemm_workspace_bytes(int M, int N, int K, int x_bits, int w_bits, int
 {
     (void)x_bits;
     (void)w_bits;
+    const size_t need = gemm_scratch_bytes(M, N, K, route);
+    return need ? need + ABQ_WORKSPACE_COUNTER_BYTES : 0;
+}
+
+} // extern "C"
+
+size_t abq::gemm_scratch_bytes(int M, int N, int K, int route)
+{
     size_t need = 0;
     if (route == ABQ_ROUTE_AUTO || route == ABQ_ROUTE_I8_MMA) // AUTO may take this route at any M (per-group scales)
         need = decode_workspace_bytes(M, N, K);
@@ -155,6 +163,8 @@ size_t abq_gemm_workspace_bytes(int M, int N, int K, int x_bits, int w_bits, int
     }
     return (need + 255) & ~(size_t)255;
 }
+
+extern "C" {
 
 size_t abq_gemm_prepared_weight_bytes(const abq_gemm_params *params)
 {

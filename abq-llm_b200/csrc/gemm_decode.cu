@@ -17,20 +17,24 @@ static int device_sms()
     return 148;
 }
 
-// Workspace (only used when K is split over CTAs): [tile counters][partial slots for kDecodeMaxSlices slices]
-void decode_workspace_layout(int M, int N, size_t *off_partials, size_t *total)
+// Workspace (only used when K is split over CTAs): [tile counters][partial slots for kDecodeMaxSlices slices].  The slots start behind
+// the room that all plans leave to counters (another plan's may reach further than this one's), in a workspace that has it.
+void decode_workspace_layout(int M, int N, size_t bytes, size_t *off_partials, size_t *total)
 {
     const int tiles = (N + 15) / 16;
     const int rows = M < 16 ? M : 16; // taller problems run as launches of 16 rows, one after the other
+    const size_t slots = (size_t)kDecodeMaxSlices * tiles * rows * 16 * 4;
     *off_partials = ((size_t)tiles * 4 + 255) & ~(size_t)255;
-    *total = *off_partials + (size_t)kDecodeMaxSlices * tiles * rows * 16 * 4;
+    if (*off_partials < ABQ_WORKSPACE_COUNTER_BYTES && bytes >= ABQ_WORKSPACE_COUNTER_BYTES + slots)
+        *off_partials = ABQ_WORKSPACE_COUNTER_BYTES;
+    *total = *off_partials + slots;
 }
 
 size_t decode_workspace_bytes(int M, int N, int K)
 {
     (void)K;
     size_t a, total;
-    decode_workspace_layout(M, N, &a, &total);
+    decode_workspace_layout(M, N, 0, &a, &total);
     return total;
 }
 
@@ -108,7 +112,7 @@ static bool make_layout(const abq_gemm_params &p, DecodeLayout *L)
     L->stages_per_split = (sps + best_split - 1) / best_split;
     L->ring = ring;
     L->smem = fixed + (size_t)sps * 4 * rec + (size_t)NW * ring * stage_bytes;
-    decode_workspace_layout(p.M, p.N, &L->off_partials, &L->bytes);
+    decode_workspace_layout(p.M, p.N, p.workspace_bytes, &L->off_partials, &L->bytes);
     return L->smem <= 227 * 1024;
 }
 
@@ -171,7 +175,7 @@ cudaError_t decode_launch(const abq_gemm_state *st, cudaStream_t stream)
     const abq_gemm_params &p = st->p;
     const int MT = (p.M < 16 ? p.M : 16) <= 8 ? 1 : 2; // as planned: by the rows of a full launch
     size_t off_partials, total;
-    decode_workspace_layout(p.M, p.N, &off_partials, &total);
+    decode_workspace_layout(p.M, p.N, p.workspace_bytes, &off_partials, &total);
     uint8_t *ws = reinterpret_cast<uint8_t *>(p.workspace);
     const int tiles = (p.N + 15) / 16;
     DecodeArgs a;

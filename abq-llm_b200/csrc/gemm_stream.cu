@@ -275,7 +275,7 @@ static bool make_plan(const abq_gemm_params &p, StreamPlan *P, size_t *smem_byte
     if (p.M > 16 && env_int("ABQ_STREAM_ROWS32", 0) != 0 && make_plan_rows(p, p.M < 32 ? p.M : 32, P, smem_bytes)) {
         // a K split parks 32-row partial tiles in the workspace, which callers size for 16-row launches: take it only if they fit
         size_t off_partials, total;
-        decode_workspace_layout(p.M, p.N, &off_partials, &total);
+        decode_workspace_layout(p.M, p.N, p.workspace_bytes, &off_partials, &total);
         const size_t need = off_partials + (size_t)P->slices * ((p.N + 15) / 16) * 32 * 16 * 4;
         if (P->slices == 1 || (p.workspace && p.workspace_bytes >= need)) {
             P->rows_per_launch = 32;
@@ -383,7 +383,7 @@ cudaError_t stream_launch(const abq_gemm_state *st, cudaStream_t stream)
     a.partials = nullptr;
     if (P.slices > 1) {
         size_t off_partials, total;
-        decode_workspace_layout(p.M, p.N, &off_partials, &total);
+        decode_workspace_layout(p.M, p.N, p.workspace_bytes, &off_partials, &total);
         a.counters = reinterpret_cast<int *>(p.workspace);
         a.partials = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(p.workspace) + off_partials);
     }

@@ -92,7 +92,7 @@ namespace {
 struct TcPlan {
     int q, bt, m_tiles, n_tiles, k_blocks, chunks_per_tile, split, ctas, x_slots, a_slots, ring;
     int xpart; // the epilogue needs the token sums
-    unsigned long long off_xpart, off_counters, off_partials;
+    unsigned long long off_x, off_xpart, off_counters, off_partials;
 };
 static_assert(sizeof(TcPlan) <= sizeof(abq_gemm_state().tmap[2]), "plan words");
 
@@ -135,7 +135,7 @@ TcPlan tc_plan_of(const abq_gemm_state *st)
 
 } // namespace
 
-bool tc_plan(abq_gemm_state *st, int sms, size_t off_free, size_t end, bool expanded)
+bool tc_plan(abq_gemm_state *st, int sms, const UmmaLayout &L, bool expanded)
 {
     const abq_gemm_params &p = st->p;
     const bool grouped = p.scale_mode == ABQ_SCALE_GROUP;
@@ -150,7 +150,9 @@ bool tc_plan(abq_gemm_state *st, int sms, size_t off_free, size_t end, bool expa
     // widths); otherwise the epilogue subtracts them times the token's code sum.
     const bool has_zero = p.w_zero && p.out_dtype == ABQ_OUT_FP16 && p.scale_mode == ABQ_SCALE_CHANNEL;
     P.xpart = !grouped && q > 0 && (tc_table_order(q) ? has_zero && p.w_signed : has_zero || (p.w_signed && q < 8));
-    P.off_xpart = (off_free + 255) & ~(size_t)255;
+    P.off_x = L.x;
+    const size_t end = expanded ? L.end : L.sum; // scratch: everything behind the activation codes
+    P.off_xpart = ((expanded ? L.end : L.x + (size_t)p.M * p.K) + 255) & ~(size_t)255;
     P.off_counters = (P.off_xpart + (P.xpart ? (size_t)p.M * P.k_blocks * 4 : 0) + 255) & ~(size_t)255;
     if (P.xpart && P.off_counters > end)
         return false; // (no room for the sums beside the activation codes)
@@ -204,7 +206,7 @@ bool tc_plan(abq_gemm_state *st, int sms, size_t off_free, size_t end, bool expa
     uint8_t *ws = reinterpret_cast<uint8_t *>(p.workspace);
     const uint64_t xd[2] = { (uint64_t)p.K, (uint64_t)p.M }, xs[1] = { (uint64_t)p.K };
     const uint32_t xb[2] = { 128, (uint32_t)P.bt };
-    if (!encode_tmap(st->tmap[1], TMAP_U8, 2, ws, xd, xs, xb, TMAP_SWIZZLE_128B))
+    if (!encode_tmap(st->tmap[1], TMAP_U8, 2, ws + P.off_x, xd, xs, xb, TMAP_SWIZZLE_128B))
         return false;
     if (q > 0) {
         const uint64_t KW = (uint64_t)p.K / 32;
@@ -215,7 +217,7 @@ bool tc_plan(abq_gemm_state *st, int sms, size_t off_free, size_t end, bool expa
     } else {
         const uint64_t wd[2] = { (uint64_t)p.K, (uint64_t)p.N };
         const uint32_t wb[2] = { 128, (uint32_t)kTcRows };
-        if (!encode_tmap(st->tmap[0], TMAP_U8, 2, ws + (((size_t)p.M * p.K + 255) & ~(size_t)255), wd, xs, wb, TMAP_SWIZZLE_128B))
+        if (!encode_tmap(st->tmap[0], TMAP_U8, 2, ws + L.w, wd, xs, wb, TMAP_SWIZZLE_128B))
             return false;
     }
     std::memcpy(st->tmap[2], &P, sizeof(P));
@@ -250,7 +252,7 @@ cudaError_t tc_prepare_x(const abq_gemm_state *st, cudaStream_t stream)
     PrepareXArgs a;
     a.X = reinterpret_cast<const uint32_t *>(p.X);
     a.qscale = (p.flags & ABQ_FLAG_X_HALF) ? p.x_quant_scale : nullptr;
-    a.out = reinterpret_cast<uint4 *>(ws);
+    a.out = reinterpret_cast<uint4 *>(ws + P.off_x);
     a.runs = a.plane_words = (long)p.M * (p.K / 32);
     a.bits = p.x_bits;
     a.is_signed = p.x_signed;

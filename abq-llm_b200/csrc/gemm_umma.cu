@@ -554,20 +554,23 @@ __global__ void __launch_bounds__(256) rowsum_kernel(const uint8_t *__restrict__
 
 // ------------------------------------------------------------------------------------------- host side
 
-// workspace: [X codes M x K][W codes N x K][token sums M]
-static void umma_layout(int M, int N, int K, size_t *off_w, size_t *off_sum, size_t *total)
+static UmmaLayout layout_at(int M, int N, int K, size_t base)
 {
-    *off_w = ((size_t)M * K + 255) & ~(size_t)255;
-    *off_sum = (*off_w + (size_t)N * K + 255) & ~(size_t)255;
-    *total = *off_sum + (size_t)M * 4;
+    UmmaLayout L;
+    L.base = L.x = base;
+    L.w = (L.x + (size_t)M * K + 255) & ~(size_t)255;
+    L.sum = (L.w + (size_t)N * K + 255) & ~(size_t)255;
+    L.end = L.sum + (size_t)M * 4;
+    return L;
 }
 
-size_t umma_workspace_bytes(int M, int N, int K)
+UmmaLayout umma_layout(const abq_gemm_params &p)
 {
-    size_t a, b, t;
-    umma_layout(M, N, K, &a, &b, &t);
-    return t;
+    const UmmaLayout L = layout_at(p.M, p.N, p.K, ABQ_WORKSPACE_COUNTER_BYTES);
+    return p.workspace_bytes >= L.end ? L : layout_at(p.M, p.N, p.K, 0);
 }
+
+size_t umma_workspace_bytes(int M, int N, int K) { return layout_at(M, N, K, 0).end; }
 
 abq_status umma_plan(abq_gemm_state *st)
 {
@@ -584,9 +587,8 @@ abq_status umma_plan(abq_gemm_state *st)
         if ((size_t)scale_groups * 512 > 120 * 1024)
             return ABQ_ERR_UNSUPPORTED; // (as many groups per row as this route has always taken)
     }
-    size_t off_w, off_sum, total;
-    umma_layout(p.M, p.N, p.K, &off_w, &off_sum, &total);
-    if (!p.workspace || p.workspace_bytes < total)
+    const UmmaLayout L = umma_layout(p);
+    if (!p.workspace || p.workspace_bytes < L.end)
         return ABQ_ERR_WORKSPACE;
     if (reinterpret_cast<uintptr_t>(p.workspace) & 255)
         return ABQ_ERR_INVALID_ARG;
@@ -605,10 +607,17 @@ abq_status umma_plan(abq_gemm_state *st)
     const bool ragged = p.N % (p.out_dtype == ABQ_OUT_INT32 ? 4 : 8) != 0;
     const int planes_rows = env_int("ABQ_TC_ROWS", grouped ? 128 : (ragged ? 4096 : 256));
     const bool pairs_asked = env_int("ABQ_UMMA_PAIRS", 0) != 0;
-    if (!(p.flags & ABQ_FLAG_WEIGHTS_PREPARED) && !pairs_asked && p.M <= planes_rows && tc_plan(st, sms, off_w, off_sum, false))
-        return ABQ_OK;
+    if (!(p.flags & ABQ_FLAG_WEIGHTS_PREPARED) && !pairs_asked && p.M <= planes_rows) {
+        // (these plans use the weight codes' place as scratch only: the counters' room may come out of that)
+        UmmaLayout S = L;
+        S.x = ABQ_WORKSPACE_COUNTER_BYTES;
+        if ((S.x == L.x || S.x + (size_t)p.M * p.K <= L.sum) && tc_plan(st, sms, S, false))
+            return ABQ_OK;
+        if (S.x != L.x && tc_plan(st, sms, L, false))
+            return ABQ_OK;
+    }
     if (grouped)
-        return tc_plan(st, sms, total, total, true) ? ABQ_OK : ABQ_ERR_UNSUPPORTED;
+        return tc_plan(st, sms, L, true) ? ABQ_OK : ABQ_ERR_UNSUPPORTED;
     // N tile: the persistent CTAs run ceil(tiles / SMs) tiles each.  Narrower tiles balance better, but measured per
     // output column they cost almost twice as much (operand fetch per operation doubles), so they only win on small grids
     const int m_tiles = (p.M + kUmmaBM - 1) / kUmmaBM;
@@ -645,8 +654,8 @@ abq_status umma_plan(abq_gemm_state *st)
     const uint64_t dims_a[2] = { (uint64_t)p.K, (uint64_t)p.M }, dims_b[2] = { (uint64_t)p.K, (uint64_t)p.N };
     const uint64_t strides[1] = { (uint64_t)p.K };
     const uint32_t box_a[2] = { (uint32_t)kUmmaBK, (uint32_t)kUmmaBM }, box_b[2] = { (uint32_t)kUmmaBK, (uint32_t)(paired ? kPairBN / 2 : BN) };
-    if (!encode_tmap(st->tmap[0], TMAP_U8, 2, ws, dims_a, strides, box_a, TMAP_SWIZZLE_128B) ||
-        !encode_tmap(st->tmap[1], TMAP_U8, 2, ws + off_w, dims_b, strides, box_b, TMAP_SWIZZLE_128B))
+    if (!encode_tmap(st->tmap[0], TMAP_U8, 2, ws + L.x, dims_a, strides, box_a, TMAP_SWIZZLE_128B) ||
+        !encode_tmap(st->tmap[1], TMAP_U8, 2, ws + L.w, dims_b, strides, box_b, TMAP_SWIZZLE_128B))
         return ABQ_ERR_CUDA;
     long tiles = (long)m_tiles * ((p.N + BN - 1) / BN);
     if (paired) { // 256-row tiles, two CTAs each
@@ -730,18 +739,16 @@ static int folded_group(const abq_gemm_params &p) { return p.scale_mode == ABQ_S
 cudaError_t umma_prepare_weights(const abq_gemm_state *st, cudaStream_t stream)
 {
     const abq_gemm_params &p = st->p;
-    size_t off_w, off_sum, total;
-    umma_layout(p.M, p.N, p.K, &off_w, &off_sum, &total);
-    return unpack_i8(reinterpret_cast<const uint32_t *>(p.W), reinterpret_cast<uint8_t *>(p.workspace) + off_w, p.N, p.K, p.w_bits, p.w_signed,
-                     stream, folded_zero(p), folded_group(p));
+    return unpack_i8(reinterpret_cast<const uint32_t *>(p.W), reinterpret_cast<uint8_t *>(p.workspace) + umma_layout(p).w, p.N, p.K, p.w_bits,
+                     p.w_signed, stream, folded_zero(p), folded_group(p));
 }
 
 cudaError_t umma_launch(const abq_gemm_state *st, cudaStream_t stream)
 {
     const abq_gemm_params &p = st->p;
-    size_t off_w, off_sum, total;
-    umma_layout(p.M, p.N, p.K, &off_w, &off_sum, &total);
-    uint8_t *ws = reinterpret_cast<uint8_t *>(p.workspace);
+    const UmmaLayout L = umma_layout(p);
+    uint8_t *xc = reinterpret_cast<uint8_t *>(p.workspace) + L.x, *wc = reinterpret_cast<uint8_t *>(p.workspace) + L.w;
+    int *sums = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(p.workspace) + L.sum);
     cudaError_t e;
     const bool tc = tc_planned(st);
     if (tc && !tc_expanded(st))
@@ -749,15 +756,14 @@ cudaError_t umma_launch(const abq_gemm_state *st, cudaStream_t stream)
     else if (p.flags & ABQ_FLAG_X_HALF) { // fp16 activations: quantise straight to codes; weights as usual
         e = cudaSuccess;
         if (!(p.flags & ABQ_FLAG_WEIGHTS_PREPARED))
-            e = unpack_i8(reinterpret_cast<const uint32_t *>(p.W), ws + off_w, p.N, p.K, p.w_bits, p.w_signed, stream, folded_zero(p),
-                          folded_group(p));
+            e = unpack_i8(reinterpret_cast<const uint32_t *>(p.W), wc, p.N, p.K, p.w_bits, p.w_signed, stream, folded_zero(p), folded_group(p));
         if (e == cudaSuccess)
-            e = quantize_codes(p.X, p.x_quant_scale, ws, p.M, p.K, p.x_bits, stream);
+            e = quantize_codes(p.X, p.x_quant_scale, xc, p.M, p.K, p.x_bits, stream);
     } else if (p.flags & ABQ_FLAG_WEIGHTS_PREPARED) // the weight codes are in place: expand the activations only
-        e = unpack_i8(reinterpret_cast<const uint32_t *>(p.X), ws, p.M, p.K, p.x_bits, p.x_signed, stream);
+        e = unpack_i8(reinterpret_cast<const uint32_t *>(p.X), xc, p.M, p.K, p.x_bits, p.x_signed, stream);
     else
-        e = unpack_pair_i8(reinterpret_cast<const uint32_t *>(p.X), ws, p.M, p.x_bits, p.x_signed, reinterpret_cast<const uint32_t *>(p.W),
-                           ws + off_w, p.N, p.w_bits, p.w_signed, p.K, stream, folded_zero(p), folded_group(p));
+        e = unpack_pair_i8(reinterpret_cast<const uint32_t *>(p.X), xc, p.M, p.x_bits, p.x_signed, reinterpret_cast<const uint32_t *>(p.W), wc, p.N,
+                           p.w_bits, p.w_signed, p.K, stream, folded_zero(p), folded_group(p));
     if (e != cudaSuccess)
         return e;
     if (tc)
@@ -765,11 +771,11 @@ cudaError_t umma_launch(const abq_gemm_state *st, cudaStream_t stream)
     UmmaArgs a;
     a.xsum = nullptr;
     if (p.scale_mode == ABQ_SCALE_CHANNEL && p.w_zero && !folded_zero(p)) {
-        rowsum_kernel<<<(p.M + 7) / 8, 256, 0, stream>>>(ws, reinterpret_cast<int *>(ws + off_sum), p.M, p.K, p.x_signed);
+        rowsum_kernel<<<(p.M + 7) / 8, 256, 0, stream>>>(xc, sums, p.M, p.K, p.x_signed);
         e = cudaGetLastError();
         if (e != cudaSuccess)
             return e;
-        a.xsum = reinterpret_cast<const int *>(ws + off_sum);
+        a.xsum = sums;
     }
     a.M = p.M;
     a.N = p.N;

@@ -54,7 +54,7 @@ extern "C" abq_status abq_gemm_static_scratch(const abq_gemm_params *params, abq
     // workspace for split-K partial sums only, so that combination, asked for by name, is served.
     if ((params->flags & ABQ_FLAG_WEIGHTS_PREPARED) && !(params->route == ABQ_ROUTE_I8_MMA && params->w_prepared))
         return ABQ_ERR_INVALID_ARG;
-    const size_t need = abq_gemm_workspace_bytes(params->M, params->N, params->K, params->x_bits, params->w_bits, params->route);
+    const size_t need = abq::gemm_scratch_bytes(params->M, params->N, params->K, params->route); // (one-shot calls clear their counters)
     if (need > (size_t)ABQ_STATIC_SCRATCH_BYTES)
         return ABQ_ERR_WORKSPACE; // the problem needs more scratch than the built-in array holds: use abq_gemm with a workspace
     void *scratch = nullptr;

@@ -143,7 +143,7 @@ typedef struct abq_gemm_params {
     const float *x_scale;   /* optional per-token fp32 scale [M], NULL = 1 */
     int route;              /* abq_route */
     int flags;              /* ABQ_FLAG_* */
-    void *workspace;        /* >= abq_gemm_workspace_bytes(), 256-byte aligned */
+    void *workspace;        /* >= abq_gemm_workspace_bytes() (ABQ_WORKSPACE_COUNTER_BYTES less where no other plan shares it), 256-byte aligned */
     size_t workspace_bytes;
     int *status_word;       /* optional device int, set non-zero by a kernel whose bounded wait expired */
     const float *x_quant_scale; /* ABQ_FLAG_X_HALF: device float, the static activation scale */
@@ -172,14 +172,19 @@ typedef struct abq_gemm_state {
     abq_fused_allreduce ar;         /* copy of *p.allreduce (world == 0: none) */
 } abq_gemm_state;
 
-/* Bytes of caller-owned scratch a GEMM of this shape may need (route AUTO: the maximum over routes). */
+/* Bytes of caller-owned scratch a GEMM of this shape may need (route AUTO: the maximum over routes).  The first
+ * ABQ_WORKSPACE_COUNTER_BYTES belong to the arrival counters of plans that split K over CTAs (4 bytes per 16 output features, so
+ * up to 1 Mi features); other plans leave them alone, which is what lets plans share a workspace. */
+#define ABQ_WORKSPACE_COUNTER_BYTES ((size_t)256 << 10)
 ABQ_API size_t abq_gemm_workspace_bytes(int M, int N, int K, int x_bits, int w_bits, int route);
 
 /*
  * Plan a GEMM: validates, picks the route and tile, encodes TMA descriptors.  Host work, except that a
  * decode-shape plan which splits K over CTAs clears its arrival counters (the first 4 * ceil(N / 16) bytes of the
  * workspace) and waits for that: call it outside stream capture and not while a GEMM on the same workspace is
- * running; launches leave the counters cleared, so plans may share a workspace.  Replaces `AqBMMAInitFn_t` / `AqBWMMAInitFn_t`
+ * running.  Launches leave the counters cleared, so plans of any sizes and row counts may share a workspace, one launch after
+ * the other, if each of them is given all of it and it holds the largest abq_gemm_workspace_bytes() among them (not: a plan whose
+ * prepared weights live in it, see ABQ_FLAG_WEIGHTS_PREPARED).  Replaces `AqBMMAInitFn_t` / `AqBWMMAInitFn_t`
  * (engine/mma_any/aq_bmma_op.h:141-151,163; aq_wmma_op.h) and the per-config
  * `AqBMMA_..._InitFn` globals (engine/common/base.h:144-166): tile shape is chosen here, not by name.
  */
@@ -316,8 +321,8 @@ ABQ_API abq_status abq_unpack_int8(const void *planes, void *out_i8, int rows, i
  * cudaFree, no allocating library routine), which is what a caller needs that runs inside a stream-ordered forward
  * pass with a workspace it does not size itself (the FasterTransformer linear layers give the GEMM wrapper only
  * x_bits * tokens * K / 8 bytes) and must not synchronise the device.
- *   - Problems whose abq_gemm_workspace_bytes() exceeds ABQ_STATIC_SCRATCH_BYTES are rejected with
- *     ABQ_ERR_WORKSPACE; use abq_gemm with a caller-owned workspace for those.
+ *   - Problems whose abq_gemm_workspace_bytes(), less ABQ_WORKSPACE_COUNTER_BYTES, exceeds ABQ_STATIC_SCRATCH_BYTES are
+ *     rejected with ABQ_ERR_WORKSPACE; use abq_gemm with a caller-owned workspace for those.
  *   - The first call on a device looks the array's address up (cudaGetSymbolAddress, with that device current).
  *     Make that first call outside any stream capture.
  *   - All calls on a device share the one array and it keeps what the last call left in it.  The kernels

@@ -6,6 +6,7 @@ import subprocess
 from pathlib import Path
 
 import pytest
+import torch
 
 ROOT = Path(__file__).resolve().parent.parent
 
@@ -104,6 +105,22 @@ def test_workspace_sizes(abq):
     big = abq.gemm_workspace_bytes(4096, 4096, 4096, 8, 8)
     assert big >= 2 * 4096 * 4096  # expanded int8 copies of both operands
     assert big > abq.STATIC_SCRATCH_BYTES
+
+
+@pytest.mark.parametrize("M,N,K,route", [(64, 512, 1024, 0), (64, 512, 1024, 3), (16, 512, 11008, 2), (300, 1000, 1152, 0), (64, 16, 128, 3)])
+def test_a_workspace_without_the_room_for_sharing_is_still_taken(abq, M, N, K, route):
+    """The room for other plans' counters is asked for, not required: without it a plan is made (as far as that goes without a
+    device: the next step, TMA descriptors or clearing counters, is a CUDA call), with less it is refused."""
+    from abq_llm_b200 import binding as B
+    p, st = B.GemmParams(), B.GemmState()
+    p.M, p.N, p.K, p.x_bits, p.w_bits, p.route = M, N, K, 4, 4, route
+    p.X = p.W = p.D = p.workspace = 4096
+    full = abq.gemm_workspace_bytes(M, N, K, 4, 4, route)
+    if torch.cuda.is_available():
+        pytest.skip("the addresses are not device memory")
+    for nbytes, status in ((full, 4), (full - abq.WORKSPACE_COUNTER_BYTES, 4), (full - abq.WORKSPACE_COUNTER_BYTES - 512, 3)):
+        p.workspace_bytes = nbytes
+        assert abq.lib().abq_gemm_init(ctypes.byref(p), ctypes.byref(st)) == status, nbytes
 
 
 def test_missing_library_fails_loudly(abq, monkeypatch, tmp_path):
