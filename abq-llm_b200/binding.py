@@ -189,10 +189,12 @@ def gemm_prepared_weight_bytes(params: GemmParams) -> int:
 
 
 def state_kernel(state: GemmState) -> str:
-    """Name of the GEMM kernel a plan launches (for reports): the route, and on the decode route which of its two kernels."""
+    """Name of the GEMM kernel a plan launches (for reports): the route, and which of the route's kernels."""
     if state.route == ROUTE_I8_MMA:
         return "stream_kernel" if (state.tmap[1][0] & 0xffffffff) == 0x5354524d else "decode_kernel"
-    return {ROUTE_B1_MMA: "b1_kernel", ROUTE_I8_UMMA: "umma_kernel"}.get(state.route, "?")
+    if state.route == ROUTE_I8_UMMA:  # tc_kernel reads the weights as planes, or (codes) as the int8 expansion in the workspace
+        return {0: "umma_kernel", 2: "umma2_kernel", 3: "tc_kernel", 4: "tc_kernel (codes)"}.get(state.tile[2], "?")
+    return "b1_kernel" if state.route == ROUTE_B1_MMA else "?"
 
 
 def gemm_init(params: GemmParams) -> GemmState:

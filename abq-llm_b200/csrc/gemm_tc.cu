@@ -96,6 +96,7 @@ struct TcPlan {
 };
 static_assert(sizeof(TcPlan) <= sizeof(abq_gemm_state().tmap[2]), "plan words");
 
+constexpr int kTcPlanes = 3, kTcCodes = 4; // tile[2] of a plan: which form of the kernel (0 and 2: umma_kernel, umma2_kernel)
 constexpr size_t kTcSmem = 222 * 1024;
 
 size_t tc_smem(int q, int bt, int x_slots, int a_slots, int ring)
@@ -229,8 +230,8 @@ bool tc_plan(abq_gemm_state *st, int sms, const UmmaLayout &L, bool expanded)
     st->cluster = 1;
     st->shared_mem_size = tc_smem(q, P.bt, P.x_slots, P.a_slots, P.ring);
     st->tile[0] = kTcRows;
-    st->tile[1] = P.x_slots;
-    st->tile[2] = 3;
+    st->tile[1] = P.split;
+    st->tile[2] = expanded ? kTcCodes : kTcPlanes;
     st->tile[3] = P.bt;
     return true;
 }
@@ -240,9 +241,9 @@ static bool tc_folds_zero(const abq_gemm_params &p, const TcPlan &P)
     return p.w_zero && p.out_dtype == ABQ_OUT_FP16 && !p.w_signed && (p.scale_mode == ABQ_SCALE_GROUP || (p.scale_mode == ABQ_SCALE_CHANNEL && tc_table_order(P.q)));
 }
 
-bool tc_planned(const abq_gemm_state *st) { return st->tile[2] == 3; }
+bool tc_planned(const abq_gemm_state *st) { return st->tile[2] == kTcPlanes || st->tile[2] == kTcCodes; }
 
-bool tc_expanded(const abq_gemm_state *st) { return tc_plan_of(st).q == 0; }
+bool tc_expanded(const abq_gemm_state *st) { return st->tile[2] == kTcCodes; }
 
 cudaError_t tc_prepare_x(const abq_gemm_state *st, cudaStream_t stream)
 {

@@ -90,3 +90,14 @@ def test_scales_of_groups_of_64_off_a_word(abq, oracle, cuda, M):
         got.append(d)
     check_close(got[0], oracle.dequant_gemm(x, w, aligned.cpu().numpy(), zero.astype(np.int32), tok, group))
     assert np.array_equal(got[0].view(np.uint16), got[1].view(np.uint16))
+
+
+@pytest.mark.parametrize("M,N,group,want", [(32, 4096, 0, "tc_kernel"), (200, 256, 0, "tc_kernel"), (512, 256, 0, "umma_kernel"), (512, 257, 0, "tc_kernel"),
+                                            (100, 256, 64, "tc_kernel"), (200, 256, 128, "tc_kernel (codes)")])
+def test_the_kernel_a_plan_reports(abq, oracle, cuda, M, N, group, want):
+    K = 4096
+    rng = np.random.default_rng(N)
+    kw = dict(out_fp16=True, scale_mode=abq.SCALE_GROUP, group_size=group, w_scale=dev(np.ones((N, K // group), dtype=np.float16))) if group else {}
+    _, st = run_gemm(abq, planes_dev(oracle, rand_codes(rng, M, K, 2, True), 2), planes_dev(oracle, rand_codes(rng, N, K, 2, False), 2), M, N, K,
+                     x_bits=2, w_bits=2, x_signed=True, w_signed=False, **kw)
+    assert abq.state_kernel(st) == want
