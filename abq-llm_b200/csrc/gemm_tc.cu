@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(128) prepare_x_kernel(const PrepareXArgs a)
 namespace {
 
 struct TcPlan {
-    int q, bt, m_tiles, n_tiles, k_blocks, chunks_per_tile, split, ctas, x_slots, a_slots, ring;
+    int q, bt, m_tiles, n_tiles, k_blocks, chunk_blocks, chunks_per_tile, split, ctas, x_slots, a_slots, ring;
     int xpart; // the epilogue needs the token sums
     unsigned long long off_x, off_xpart, off_counters, off_partials;
 };
@@ -145,7 +145,10 @@ bool tc_plan(abq_gemm_state *st, int sms, const UmmaLayout &L, bool expanded)
     P.q = q;
     P.k_blocks = p.K / 128;
     const int ck = tc_chunk_blocks(q);
-    P.chunks_per_tile = (P.k_blocks + ck - 1) / ck;
+    P.chunk_blocks = ck;
+    while (grouped && p.group_size > 128 && P.chunk_blocks % (p.group_size / 128)) // groups wider than 128 stay whole
+        P.chunk_blocks += ck;
+    P.chunks_per_tile = (P.k_blocks + P.chunk_blocks - 1) / P.chunk_blocks;
     P.n_tiles = (p.N + kTcRows - 1) / kTcRows;
     // Zero points and the offset of signed codes: subtracted by the expanders with scale groups and where that is free (the table
     // widths); otherwise the epilogue subtracts them times the token's code sum.
@@ -187,7 +190,7 @@ bool tc_plan(abq_gemm_state *st, int sms, const UmmaLayout &L, bool expanded)
             int x_slots, a_slots, ring;
             if (!tc_buffers(q, grouped, bt, &x_slots, &a_slots, &ring))
                 continue;
-            const double rounds = split ? (double)chunks * ck / ctas : (double)((tiles + ctas - 1) / ctas) * P.k_blocks;
+            const double rounds = split && P.chunk_blocks > ck ? (double)((chunks + ctas - 1) / ctas) * P.chunk_blocks : split ? (double)chunks * ck / ctas : (double)((tiles + ctas - 1) / ctas) * P.k_blocks;
             const double t = rounds * block + tail + (split ? 5700.0 + 266.0 * bt : 0);
             if (best == 0 || t < best) {
                 best = t;
@@ -292,6 +295,7 @@ cudaError_t tc_launch(const abq_gemm_state *st, cudaStream_t stream)
     a.m_tiles = P.m_tiles;
     a.n_tiles = P.n_tiles;
     a.k_blocks = P.k_blocks;
+    a.chunk_blocks = P.chunk_blocks;
     a.chunks_per_tile = P.chunks_per_tile;
     a.split = P.split;
     const int chunks = P.m_tiles * P.n_tiles * P.chunks_per_tile;

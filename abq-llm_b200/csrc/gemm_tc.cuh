@@ -25,6 +25,8 @@
 // Scale groups (GROUPED): every 64 or 128 features have an accumulator of their own; the epilogue warps drain two per hand-over into
 // fp32 while the next two are multiplied.  An accumulator starts from the bits of 1.5 * 2^23 (2^23 for sums that cannot be
 // negative), so what comes back is a float already: one packed subtraction and one packed multiply-add per two elements.
+// Groups wider than 128 are summed as a whole in one int32 accumulator (beyond that start's bound) and converted once; K is then
+// cut between groups only.
 #pragma once
 #include <cuda.h>
 #include <cstring>
@@ -41,7 +43,8 @@ struct TcArgs {
     int bt;                 // tokens per tile
     int m_tiles, n_tiles;
     int k_blocks;           // K / 128
-    int chunks_per_tile;    // ceil(k_blocks / K blocks per chunk)
+    int chunk_blocks;       // split: K blocks per piece of work (whole plane chunks and whole scale groups)
+    int chunks_per_tile;    // ceil(k_blocks / chunk_blocks)
     int split;              // 0: whole tiles, round-robin; 1: equal runs of K chunks
     int range_q, range_r;   // split: chunks per CTA, the first range_r CTAs take one more
     int x_slots, a_slots, ring; // activation codes, expanded weight codes, plane chunks
@@ -77,7 +80,6 @@ __host__ __device__ constexpr int tc_chunk_bytes(int q) { return q * kTcRows * t
 struct TcSegment {
     int tile, m0, n0, k0, k1; // K blocks [k0, k1) of the tile at token m0, feature n0
 };
-template <int CK>
 struct TcWalk {
     int x, x1;
     __device__ __forceinline__ explicit TcWalk(const TcArgs &a)
@@ -99,8 +101,8 @@ struct TcWalk {
             s.tile = x / a.chunks_per_tile;
             const int c0 = x - s.tile * a.chunks_per_tile;
             const int c1 = min(a.chunks_per_tile, c0 + x1 - x);
-            s.k0 = c0 * CK;
-            s.k1 = min(c1 * CK, a.k_blocks);
+            s.k0 = c0 * a.chunk_blocks;
+            s.k1 = min(c1 * a.chunk_blocks, a.k_blocks);
             x += c1 - c0;
         } else {
             s.tile = x;
@@ -402,6 +404,15 @@ __device__ __forceinline__ void tc_epilogue_float(const TcArgs &a, const TcSegme
     }
 }
 
+// facc[0 .. 16) += scale * (the sums v), whole numbers
+__device__ __forceinline__ void tc_scale_add_int(const int (&v)[16], uint64_t scale2, uint64_t *facc)
+{
+#pragma unroll
+    for (int j = 0; j < 16; j += 2) {
+        const uint64_t t = pack2(__float_as_uint(__int2float_rn(v[j])), __float_as_uint(__int2float_rn(v[j + 1])));
+        facc[j / 2] = fma2(t, scale2, facc[j / 2]);
+    }
+}
 // facc[0 .. 16) += scale * (the sums v): v are accumulators that started from the bits of a power of two, i.e. read as floats they
 // are that power plus the sum
 __device__ __forceinline__ void tc_scale_add(const int (&v)[16], uint64_t minus_magic2, uint64_t scale2, uint64_t *facc)
@@ -471,7 +482,7 @@ __global__ void __launch_bounds__((4 + E + EW) * 32, 1)
     if (!(Q > 0 && warp == 2))
         pdl_wait_prior_grid(); // everything but the weight planes comes from (or goes to) what earlier kernels touch
 
-    TcWalk<CK> walk(a);
+    TcWalk walk(a);
     TcSegment sg;
     bool ok = true;
     if (warp == 0) {
@@ -500,14 +511,17 @@ __global__ void __launch_bounds__((4 + E + EW) * 32, 1)
             // (addresses in the descriptors' 16-byte units: this thread's instructions are on the critical path of every block)
             const uint64_t desc0 = make_smem_desc_sw128(0);
             const uint32_t x_base = smem_u32(smem) >> 4, a_base = smem_u32(a_ring) >> 4, x_step = (uint32_t)x_bytes_slot >> 4;
+            const int wide = GROUPED && a.group_size > 128 ? a.group_size >> 7 : 0; // K blocks per group, 0: groups of at most one block
+            int open = 0;                                                           // wide: blocks that the open group still misses
             while (ok && walk.next(a, sg)) {
                 int b = 0;
                 uint32_t acc = 0;
                 for (int kb = sg.k0; ok && kb < sg.k1; ++kb) {
                     // ungrouped: one accumulator per tile; grouped: two per hand-over (two 64-feature groups of a K block,
-                    // or two K blocks)
-                    const bool fresh = GROUPED ? (a.group_size == 64 || ((kb - sg.k0) & 1) == 0) : kb == sg.k0;
+                    // or two K blocks), or one per wide group
+                    const bool fresh = !GROUPED ? kb == sg.k0 : wide ? open == 0 : a.group_size == 64 || ((kb - sg.k0) & 1) == 0;
                     if (fresh) {
+                        open = wide; // (a segment holds whole groups)
                         b = unit & 1;
                         // (grouped: the epilogue hands the accumulators over with the starting value in them, the first time too)
                         ok = mbar_wait_bounded(&acc_empty[b], ((unit >> 1) & 1) ^ (GROUPED ? 0 : 1), a.status, STATUS_TIMEOUT_PIPE);
@@ -524,21 +538,21 @@ __global__ void __launch_bounds__((4 + E + EW) * 32, 1)
                     tmem_fence_after();
                     const uint32_t sx = x_base + s * x_step;
                     const uint64_t db = desc0 + sx, da = desc0 + (Q > 0 ? a_base + c * (kTcABytes >> 4) : sx + a.bt * 8);
-                    if (GROUPED && a.group_size == 64) {
+                    if (!GROUPED || wide) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            umma_i8(acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), a.idesc, !(fresh && k == 0));
+                        if (GROUPED ? --open == 0 : kb + 1 == sg.k1)
+                            umma_commit(&acc_full[b]);
+                    } else if (a.group_size == 64) {
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
                             umma_i8(acc + (uint32_t)((k >> 1) * a.bt), da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), a.idesc, 1);
-                    } else if (GROUPED) {
+                    } else {
                         const int half = (kb - sg.k0) & 1;
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
                             umma_i8(acc + (uint32_t)(half * a.bt), da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), a.idesc, 1);
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            umma_i8(acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), a.idesc, !(kb == sg.k0 && k == 0));
-                        if (kb + 1 == sg.k1)
-                            umma_commit(&acc_full[b]);
                     }
                     umma_commit(&done[j % kTcDone]);
                     ++j;
@@ -724,8 +738,28 @@ __global__ void __launch_bounds__((4 + E + EW) * 32, 1)
                 // groups of 64: an even number of them per row, so a K block's two lie in one word -- where the array starts on one
                 // (a caller's view into a larger fp16 buffer need not)
                 const bool scale_words = (reinterpret_cast<uintptr_t>(a.w_scale) & 3) == 0;
-                const int units = g64 ? sg.k1 - sg.k0 : (sg.k1 - sg.k0 + 1) >> 1;
-                // the scale group of accumulator h of unit u (groups of at least a K block)
+                const int units = a.group_size > 128 ? 0 : g64 ? sg.k1 - sg.k0 : (sg.k1 - sg.k0 + 1) >> 1;
+                for (int kb = sg.k0; a.group_size > 128 && kb < sg.k1; kb += a.group_size >> 7, ++unit) {
+                    const int b = unit & 1;
+                    const uint32_t u0 = __float_as_uint(__half2float(ld_half(srow + tc_group_of(a, kb))));
+                    ok = tc_wait(&acc_full[b], (unit >> 1) & 1, a, STATUS_TIMEOUT_MMA);
+                    if (!ok)
+                        break;
+                    tmem_fence_after();
+                    const uint32_t taddr = tlane + (uint32_t)(2 * b * a.bt + share * COLS);
+#pragma unroll
+                    for (int i = 0; i < NCH; ++i) {
+                        int v[CH];
+                        tmem_ld16_nowait(taddr + (uint32_t)(i * CH), v);
+                        tmem_ld_wait();
+                        tc_scale_add_int(v, pack2(u0, u0), facc + i * (CH / 2));
+                    }
+                    tmem_fence_before();
+                    __syncwarp();
+                    if (lane == 0)
+                        mbar_arrive(&acc_empty[b]);
+                }
+                // the scale group of accumulator h of unit u (groups of at most a K block)
                 auto group_of = [&](int u, int h) { return tc_group_of(a, min(sg.k0 + 2 * u + h, sg.k1 - 1)); };
                 auto fetch = [&](int u) -> __half2 {
                     if (g64 && scale_words)

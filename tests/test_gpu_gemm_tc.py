@@ -101,3 +101,30 @@ def test_the_kernel_a_plan_reports(abq, oracle, cuda, M, N, group, want):
     _, st = run_gemm(abq, planes_dev(oracle, rand_codes(rng, M, K, 2, True), 2), planes_dev(oracle, rand_codes(rng, N, K, 2, False), 2), M, N, K,
                      x_bits=2, w_bits=2, x_signed=True, w_signed=False, **kw)
     assert abq.state_kernel(st) == want
+
+
+@pytest.mark.parametrize("split", [0, 1])
+@pytest.mark.parametrize("M,N,K,group", [(16, 1024, 4096, 256), (16, 1024, 4096, 1024), (16, 2048, 3840, 640), (100, 300, 3072, 3072), (200, 300, 1536, 512),
+                                         (16, 1024, 4096, 4096)])
+def test_wide_groups_are_summed_whole(abq, oracle, cuda, M, N, K, group, split, monkeypatch):
+    """Groups of more than 128 features are summed as whole numbers and rounded once, however K is cut.  Here the two halves of a group
+    almost cancel: the sum is 1 to 3, the halves reach 3.9e6 x group / 256, of which a product with the scale that is rounded to fp32 per 128
+    features keeps 24 bits, i.e. an error of a tenth of the result and more.  The exact sums leave the fp32 rounding of the sum over
+    groups (relative 2^-24 each, all terms positive) and of the result (2^-11)."""
+    monkeypatch.setenv("ABQ_TC_SPLIT", str(split))
+    rng = np.random.default_rng(group + M)
+    half, G = group // 2, K // group
+    x = np.empty((M, G, 2, half), dtype=np.int32)
+    w = np.empty((N, G, 2, half), dtype=np.int32)
+    x[:, :, 0] = rng.integers(120, 128, size=(M, G, half))
+    w[:, :, 0] = rng.integers(200, 256, size=(N, G, half))
+    x[:, :, 0, 0] = rng.integers(1, 4, size=(M, G))
+    x[:, :, 1], w[:, :, 1] = -x[:, :, 0], w[:, :, 0]
+    w[:, :, 1, 0] -= 1
+    x, w = x.reshape(M, K), w.reshape(N, K)
+    scale = rng.uniform(0.001, 0.02, size=(N, G)).astype(np.float16)
+    got, st = run_gemm(abq, planes_dev(oracle, x, 8), planes_dev(oracle, w, 8), M, N, K, x_bits=8, w_bits=8, x_signed=True, w_signed=False,
+                       out_fp16=True, scale_mode=abq.SCALE_GROUP, group_size=group, w_scale=dev(scale), route=abq.ROUTE_I8_UMMA)
+    assert abq.state_kernel(st) == ("tc_kernel" if M <= 128 else "tc_kernel (codes)")
+    ref = oracle.dequant_gemm(x, w, scale, None, np.ones(M, dtype=np.float32), group)
+    assert np.all(np.abs(got.astype(np.float64) - ref) <= (2.0 ** -11 + 2.0 ** -24 * (G + 2)) * np.abs(ref))
