@@ -173,6 +173,43 @@ size_t abq_gemm_prepared_weight_bytes(const abq_gemm_params *params)
     return stream_prepared_bytes(*params);
 }
 
+// 17..32 rows, no scale groups: whether two launches of the mma.sync route beat the tensor-core kernel over planes as planned in `st`.
+// Measured over 22 matrices from 3000 x 1536 to 32000 x 512 and 512 x 16384, 1 to 8 bits, 17 to 32 rows, with fp16 activations (with
+// and without ABQ_FLAG_PDL) and with planes, weights out of HBM; us, two launches -> one.  From 4 Mi weights on one launch is the rule
+// (4096 x 4096 W2 15.9 -> 13.3 at 17 rows, W4 20.7 -> 14.3 at 32; 12288 x 4096 W8 46.8 -> 23.5; 2048 x 4096 W4 12.9 -> 11.8 at 17;
+// 7168 x 1536 W4 11.0 -> 9.2), but for
+//   * long rows that the plan could not cut over CTAs (too little scratch for the pieces), up to 24 rows or with 8 bits: 1024 x 4096
+//     W8 15.5 -> 20.4 at 17, 19.8 -> 20.4 at 32; W5 17.5 -> 17.9 at 17, but 21.8 -> 17.9 at 32.  Or of very few features, where many
+//     pieces make a tile: 512 x 11008 W5 21.4 -> 23.8 at 17
+//   * rows of medium length and few features, i.e. few whole tiles of 16 to 32 K blocks, up to some row count (the second launch gets
+//     heavier with its rows).  fp16 activations, which every CTA of the mma.sync route quantises for itself: never without PDL (2560 x
+//     2560 W4 14.4 -> 13.5 at 20), with it up to 20 (3072 x 3072 W4 12.6 -> 13.0 at 20, 13.3 -> 12.7 at 24); planes: up to 28
+//     (2560 x 2560 W4 12.0 -> 12.6 at 20, 13.1 -> 12.6 at 32; below 6 Mi always: 2048 x 2048 W4 9.1 -> 10.2 at 32)
+//   * five bits until 9 Mi (2560 x 2560 11.9 -> 13.3, 3072 x 3072 18.7 -> 14.8; planes 4096 x 2048 11.4 -> 12.7), seven and eight of such
+//     rows until 6 Mi (2048 x 2048 W8 11.6 -> 12.7, 2560 x 2560 15.3 -> 12.7), six never (16.4 -> 11.8)
+static bool two_launches_win(const abq_gemm_state &st)
+{
+    const abq_gemm_params &p = st.p;
+    const double mi = (double)p.N * p.K / (1 << 20);
+    const bool half = (p.flags & ABQ_FLAG_X_HALF) != 0, cut = st.tile[1] != 0;
+    const int q = p.w_bits;
+    if (mi < 4 || mi >= 16)
+        return mi < 4;
+    if (p.K >= 4096)
+        return (!cut && (p.M <= 24 || q == 8)) || (p.N < 1024 && p.M <= 20 && (q == 5 || q == 8));
+    if (p.K <= 1536)
+        return false;
+    if (q == 5 && !half && mi < 9)
+        return true;
+    if (p.N >= 4096)
+        return false;
+    if (q >= 5)
+        return mi < (q == 5 ? 9 : q == 6 ? 0 : 6);
+    if (half)
+        return p.M <= 20 && (p.flags & ABQ_FLAG_PDL);
+    return p.M <= 28 || mi < 6;
+}
+
 static abq_status plan_gemm(const abq_gemm_params *params, abq_gemm_state *state, bool clear_counters)
 {
     if (!params || !state)
@@ -196,8 +233,8 @@ static abq_status plan_gemm(const abq_gemm_params *params, abq_gemm_state *state
     int route = params->route;
     if (route == ABQ_ROUTE_AUTO) {
         // up to 16 rows: one launch of the mma.sync route.  17..32 rows: two such launches with scale groups (at 20 rows equal or a
-        // little faster than the tensor-core kernel) and for matrices of less than 4 Mi weights; otherwise (below) the
-        // tensor-core kernel over the planes, and always where the weight codes are already expanded.  Above: tcgen05.
+        // little faster than the tensor-core kernel) and for small matrices; otherwise (below) the tensor-core kernel over the
+        // planes, and always where the weight codes are already expanded.  Above: tcgen05.
         const int small = (params->flags & ABQ_FLAG_WEIGHTS_PREPARED) ? 16 : 32;
         route = params->M <= small ? ABQ_ROUTE_I8_MMA : ABQ_ROUTE_I8_UMMA;
     }
@@ -208,13 +245,11 @@ static abq_status plan_gemm(const abq_gemm_params *params, abq_gemm_state *state
         if (s == ABQ_ERR_UNSUPPORTED)
             route = ABQ_ROUTE_I8_MMA;
     }
-    // 17..32 rows: two launches of the mma.sync route against one of tc_kernel, W4A4, 32 rows: 12288 x 4096 27.2 -> 17.0 us,
-    // 4096 x 4096 17.8 -> 12.4, 22016 x 4096 38.2 -> 25.3, 4096 x 11008 35.3 -> 20.2.  A problem whose workspace does not hold
-    // that kernel's scratch keeps the two launches.
+    // 17..32 rows: one launch of tc_kernel instead of two of the mma.sync route, where that is faster and the workspace holds the
+    // kernel's scratch
     bool planes_kernel = false;
-    if (params->route == ABQ_ROUTE_AUTO && route == ABQ_ROUTE_I8_MMA && params->M > 16 && params->scale_mode != ABQ_SCALE_GROUP && !params->allreduce &&
-        (long long)params->N * params->K >= (4ll << 20)) {
-        planes_kernel = umma_plan(state) == ABQ_OK && tc_planned(state) && !tc_expanded(state);
+    if (params->route == ABQ_ROUTE_AUTO && route == ABQ_ROUTE_I8_MMA && params->M > 16 && params->scale_mode != ABQ_SCALE_GROUP && !params->allreduce) {
+        planes_kernel = umma_plan(state) == ABQ_OK && tc_planned(state) && !tc_expanded(state) && !two_launches_win(*state);
         if (planes_kernel)
             route = ABQ_ROUTE_I8_UMMA;
         else

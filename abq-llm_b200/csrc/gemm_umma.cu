@@ -601,8 +601,9 @@ abq_status umma_plan(abq_gemm_state *st)
     // Weights straight from their planes (tc_kernel) while the token tiles of a weight tile are few: expanding a tile once per
     // token tile inside the GEMM is then cheaper than writing and re-reading the whole expanded matrix.  W4A4, whole call, this
     // route before and now: 12288 x 4096 33.5 -> 18.9 us at 64 tokens, 35.6 -> 24.5 at 128, 40.3 -> 33.3 at 256, equal at 512.
-    // Rows of D that are not multiples of 16 bytes cost umma_kernel a store per value, tc_kernel nothing: 10007 x 2944 44.8 -> 20.5
-    // us at 128 tokens, 103 -> 48 at 512, 156 -> 113 at 1024.  With scale groups (2 bits, groups of 64) 12288 x 4096 55.1 -> 33.2 at 64
+    // Rows of D that are not multiples of 16 bytes cost umma_kernel a store per value, tc_kernel nothing: W4A4 10007 x 2944 44.8 -> 20.5
+    // us at 128 tokens, 102 -> 48 at 512, 464 -> 216 at 4096; 12289 x 4096 591 -> 261 at 4096, 1027 x 8192 34 -> 26 at 257, W8A8 4100 x
+    // 11008 295 -> 256 at 4096, the least gain of five matrices, three widths and 257 to 4096 tokens.  With scale groups (2 bits, groups of 64) 12288 x 4096 55.1 -> 33.2 at 64
     // tokens, equal at 128.  Weights that were expanded beforehand keep the kernels that read codes.
     const bool ragged = p.N % (p.out_dtype == ABQ_OUT_INT32 ? 4 : 8) != 0;
     const int planes_rows = env_int("ABQ_TC_ROWS", grouped ? 128 : (ragged ? 4096 : 256));

@@ -31,9 +31,9 @@ class Plan:
 
 @pytest.mark.parametrize("sizing", ["largest plan", "without the room for sharing"])
 def test_row_counts_in_turn(abq, oracle, cuda, sizing):
-    """Split K (16 rows), the tensor-core kernel over planes (32 rows by AUTO's rule for 4 Mi weights and more; 64) and over expanded codes
+    """Split K (16 rows), the tensor-core kernel over planes (32 rows by AUTO's rule for 16 Mi weights and more; 64) and over expanded codes
     (300) on one workspace.  In the smaller workspace only the plans over planes still keep clear of the counters."""
-    N, K, bits = 512, 11008, 4
+    N, K, bits = 1536, 11008, 4
     rng = np.random.default_rng(7)
     w = rand_codes(rng, N, K, bits, False)
     planes = planes_dev(oracle, w, bits)
