@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(NW * 32, 1) decode_kernel(const __grid_constan
                             } else {
                                 __half h;
                                 if (a.scale_mode == ABQ_SCALE_TENSOR_COMPAT) {
-                                    h = __hmul(__int2half_rn(v[mt][e]), ld_half(a.C));
+                                    h = __hmul_rn(__int2half_rn(v[mt][e]), ld_half(a.C)); // (_rn: never one instruction with the add below)
                                 } else {
                                     float f = GROUPED ? __int_as_float(v[mt][e]) : (float)v[mt][e] * __half2float(ld_half(a.w_scale + n));
                                     if (a.x_scale)

@@ -1097,7 +1097,7 @@ __global__ void __launch_bounds__(MT == 4 ? 256 : kStreamMaxWarps * 32, 1) strea
         } else {
             __half h;
             if (a.scale_mode == ABQ_SCALE_TENSOR_COMPAT) {
-                h = __hmul(__int2half_rn(v), ld_half(a.C));
+                h = __hmul_rn(__int2half_rn(v), ld_half(a.C)); // (_rn: never one instruction with the add below)
             } else {
                 float f = GROUPED ? __int_as_float(v) : (float)v * __half2float(ld_half(a.w_scale + n));
                 if (a.x_scale)

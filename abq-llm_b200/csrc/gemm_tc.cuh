@@ -227,7 +227,7 @@ __device__ __forceinline__ void tc_store_int(const TcArgs &a, const TcRow &row, 
     }
     __half h;
     if (MODE == 1) {
-        h = __hmul(__int2half_rn(v), row.cscale);
+        h = __hmul_rn(__int2half_rn(v), row.cscale); // (_rn: never one instruction with the residual's add)
     } else {
         h = __float2half_rn((float)v * row.scale * (a.x_scale ? __ldg(a.x_scale + m) : 1.f));
     }

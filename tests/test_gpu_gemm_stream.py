@@ -348,3 +348,37 @@ def test_residual_added_in_the_epilogue(abq, oracle, cuda, M, N, K, q, group, pr
                                     scale_mode=abq.SCALE_CHANNEL, w_scale=dev(np.ones(N, dtype=np.float16)), route=abq.ROUTE_I8_UMMA, workspace=wsu,
                                     residual=big))
     assert err.value.status == 2  # ABQ_ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("M,N,K,q,kernel,cut", [(1, 1024, 4096, 4, "stream_kernel", False), (16, 512, 11008, 4, "stream_kernel", None), (20, 264, 1152, 2, "stream_kernel", False),
+                                                (4, 520, 1024, 4, "decode_kernel", False), (16, 512, 11008, 4, "decode_kernel", True), (20, 4096, 4096, 4, "tc_kernel", True),
+                                                (20, 4096, 4096, 4, "tc_kernel", False)])
+def test_residual_behind_one_scale_factor(abq, oracle, cuda, M, N, K, q, kernel, cut, monkeypatch):
+    """The product with the one fp16 factor is rounded before the residual is added: the oracle's two fp16 roundings, then an fp16 add."""
+    from abq_llm_b200 import binding as B
+    if kernel == "tc_kernel":
+        monkeypatch.setenv("ABQ_TC_SPLIT", str(int(cut)))
+    rng = np.random.default_rng(M + N)
+    x, w = rand_codes(rng, M, K, 4, True), rand_codes(rng, N, K, q, False)
+    factor = np.float16(0.0123)
+    res = rng.normal(0, 1, size=(M, N)).astype(np.float16)
+    out = torch.zeros((M, N), dtype=torch.float16, device="cuda")
+    xp, wp, C, res_dev = planes_dev(oracle, x, 4), planes_dev(oracle, w, q), dev(np.array([factor])), dev(res)
+    ws = torch.empty(abq.gemm_workspace_bytes(M, N, K, 4, q), dtype=torch.uint8, device="cuda")
+    p = B.make_params(M, N, K, xp, wp, out, x_bits=4, w_bits=q, x_signed=True, w_signed=False, out_dtype=abq.OUT_FP16, scale_mode=abq.SCALE_TENSOR_COMPAT,
+                      C=C, workspace=ws, residual=res_dev, route=abq.ROUTE_AUTO if kernel == "tc_kernel" else abq.ROUTE_I8_MMA,
+                      flags=abq.FLAG_WEIGHTS_PREPARED if kernel == "stream_kernel" else 0)
+    prep = torch.empty(max(16, abq.gemm_prepared_weight_bytes(p)), dtype=torch.uint8, device="cuda")
+    if kernel == "stream_kernel":
+        p.w_prepared = prep.data_ptr()
+    st = abq.gemm_init(p)
+    assert abq.state_kernel(st) == kernel
+    if cut is not None:
+        assert bool(st.tile[1] if kernel == "tc_kernel" else st.cluster > 1) == cut
+    if kernel == "stream_kernel":
+        abq.gemm_prepare_weights(st)
+    abq.gemm_exec(st)
+    want = oracle.dequant_tensor_compat(oracle.gemm_values_blas(x, w), factor)
+    got = out.cpu().numpy()
+    assert np.isfinite(want.astype(np.float32)).all()
+    assert np.array_equal(got.view(np.uint16), (want + res).view(np.uint16)), f"{np.count_nonzero(got != want + res)} of {got.size} differ"
