@@ -503,6 +503,9 @@ __global__ void __launch_bounds__((4 + E + EW) * 32, 1)
                         s = 0;
                 }
             }
+            // Every copy has landed before the block ends: after a wait that ran out nobody else may be waiting for them.
+            for (int i = max(free_at, 0); i < free_at + a.x_slots; ++i)
+                mbar_wait_bounded(&xfull[i % a.x_slots], (i / a.x_slots) & 1, a.status, STATUS_TIMEOUT_TMA);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -566,11 +569,13 @@ __global__ void __launch_bounds__((4 + E + EW) * 32, 1)
                     }
                 }
             }
+            if (j > 0) // nothing still multiplies, and the last commit has arrived, before the block ends
+                mbar_wait_bounded(&done[(j - 1) % kTcDone], ((j - 1) / kTcDone) & 1, a.status, STATUS_TIMEOUT_MMA);
         }
         __syncwarp();
     } else if (warp == 2) {
         if (Q > 0 && elect_one()) {
-            int s = 0, ph = 1;
+            int s = 0, ph = 1, n = 0;
             while (ok && walk.next(a, sg)) {
                 for (int kb = sg.k0; kb < sg.k1; kb += CK) {
                     ok = mbar_wait_bounded(&pempty[s], ph, a.status, STATUS_TIMEOUT_PIPE);
@@ -578,12 +583,15 @@ __global__ void __launch_bounds__((4 + E + EW) * 32, 1)
                         break;
                     mbar_arrive_expect_tx(&pfull[s], kChunkBytes);
                     tma_load_3d(ring + (size_t)s * kChunkBytes, &tmap_w, kb * 4, sg.n0, 0, &pfull[s]);
+                    ++n;
                     if (++s == a.ring) {
                         s = 0;
                         ph ^= 1;
                     }
                 }
             }
+            for (int i = max(n - a.ring, 0); i < n; ++i)
+                mbar_wait_bounded(&pfull[i % a.ring], (i / a.ring) & 1, a.status, STATUS_TIMEOUT_TMA);
         }
         __syncwarp();
     } else if (E > 0 && warp >= 4 && warp < 4 + E) {
