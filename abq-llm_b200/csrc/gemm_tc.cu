@@ -167,8 +167,7 @@ bool tc_plan(abq_gemm_state *st, int sms, const UmmaLayout &L, bool expanded)
     // about five microseconds plus the last tile's columns; cutting tiles the trip of their pieces through L2, which
     // grows with the columns.
     double best = 0;
-    const int max_bt = !grouped ? 256 : force_bt ? 128 : 64; // (128 columns with scale groups leave four warps for the expansion)
-    for (int bt = grouped ? 16 : 32; bt <= (q == 0 ? 128 : max_bt); bt *= 2) {
+    for (int bt = grouped ? 16 : 32; bt <= (q == 0 ? 128 : grouped ? 64 : 256); bt *= 2) {
         if (q == 0 ? bt != 128 : (force_bt ? bt != force_bt : bt > (grouped ? 16 : 32) && p.M <= bt / 2))
             continue;
         const int m_tiles = (p.M + bt - 1) / bt;
@@ -290,7 +289,6 @@ cudaError_t tc_launch(const abq_gemm_state *st, cudaStream_t stream)
     TcArgs a = {};
     a.M = p.M;
     a.N = p.N;
-    a.K = p.K;
     a.bt = P.bt;
     a.m_tiles = P.m_tiles;
     a.n_tiles = P.n_tiles;

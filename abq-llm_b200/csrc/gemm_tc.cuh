@@ -39,7 +39,7 @@
 namespace abq {
 
 struct TcArgs {
-    int M, N, K;
+    int M, N;
     int bt;                 // tokens per tile
     int m_tiles, n_tiles;
     int k_blocks;           // K / 128
@@ -846,14 +846,14 @@ cudaError_t tc_launch_one(const CUtensorMap &tw, const CUtensorMap &tx, const Tc
 }
 
 // Warps of a launch.  The expansion of a block is one long dependent sequence per thread, so what it needs is warps: as many as the
-// registers allow beside the epilogue (whose sums take 64 registers with 128 tokens and scale groups; without them eight warps store
-// the columns of a tile twice as fast as four).
+// registers allow beside the epilogue (whose sums take 32 registers with scale groups; without them eight warps store the columns of a
+// tile twice as fast as four).  Over planes, tiles with scale groups end at 64 tokens: 128 would leave four warps for the expansion.
 struct TcWarps {
     int expand, epilogue;
 };
 __host__ __device__ constexpr TcWarps tc_warps(int q, bool grouped, int bt)
 {
-    return q == 0 ? TcWarps{ 0, 16 } : !grouped ? TcWarps{ 12, 8 } : bt <= 16 ? TcWarps{ 16, 4 } : bt <= 32 ? TcWarps{ 12, 4 } : bt <= 64 ? TcWarps{ 8, 8 } : TcWarps{ 4, 8 };
+    return q == 0 ? TcWarps{ 0, 16 } : !grouped ? TcWarps{ 12, 8 } : bt <= 16 ? TcWarps{ 16, 4 } : bt <= 32 ? TcWarps{ 12, 4 } : TcWarps{ 8, 8 };
 }
 
 template <int Q, int BT>
@@ -877,7 +877,6 @@ cudaError_t tc_launch_width(const CUtensorMap &tw, const CUtensorMap &tx, const 
         case 16: return tc_launch_grouped<Q, 16>(tw, tx, a, grid, smem, stream);
         case 32: return tc_launch_grouped<Q, 32>(tw, tx, a, grid, smem, stream);
         case 64: return tc_launch_grouped<Q, 64>(tw, tx, a, grid, smem, stream);
-        case 128: return tc_launch_grouped<Q, 128>(tw, tx, a, grid, smem, stream);
         }
         return cudaErrorInvalidValue;
     }
