@@ -10,53 +10,97 @@ from test_gpu_gemm_fp16 import check_close
 
 pytestmark = pytest.mark.gpu
 
+def plan_of(abq, st):
+    """(kernel, tokens per tile, K cut over CTAs) of a plan."""
+    return abq.state_kernel(st), st.tile[3], bool(st.tile[1])
+
+
+def force(monkeypatch, bt, split):
+    monkeypatch.setenv("ABQ_TC_BT", str(bt))
+    monkeypatch.setenv("ABQ_TC_SPLIT", str(int(split)))
+
+
 INT_CASES = [
-    # M, N, K, x_bits, w_bits, x_signed, w_signed
-    (1, 128, 128, 8, 1, True, False), (16, 130, 640, 4, 2, True, True), (17, 127, 1152, 8, 3, True, True), (32, 1000, 512, 3, 4, False, False),
-    (33, 4096, 4096, 4, 4, False, False), (64, 257, 2944, 6, 5, True, True), (65, 4100, 1408, 6, 6, True, False), (128, 384, 256, 7, 7, True, True),
-    (129, 1001, 896, 8, 8, True, True), (256, 4096, 384, 8, 8, False, False), (257, 300, 4096, 2, 8, True, False), (1024, 129, 2048, 5, 1, True, True),
+    # tokens per tile, K cut, M, N, K, x_bits, w_bits, x_signed, w_signed
+    (32, False, 1, 128, 128, 8, 1, True, False), (32, False, 16, 130, 640, 4, 2, True, True), (64, False, 17, 127, 1152, 8, 3, True, True),
+    (256, False, 32, 1000, 512, 3, 4, False, False), (32, False, 33, 4096, 4096, 4, 4, False, False), (128, False, 64, 257, 2944, 6, 5, True, True),
+    (64, False, 65, 4100, 1408, 6, 6, True, False), (128, False, 128, 384, 256, 7, 7, True, True), (256, False, 129, 1001, 896, 8, 8, True, True),
+    (256, False, 256, 4096, 384, 8, 8, False, False), (256, False, 257, 301, 4096, 2, 8, True, False), (256, False, 1024, 129, 2048, 5, 1, True, True),
+    # cut tiles: sizes whose partial tiles fit into the scratch
+    (32, True, 1, 384, 2048, 8, 1, True, False), (32, True, 17, 257, 1408, 4, 2, True, True), (32, True, 33, 1000, 8192, 8, 3, True, True),
+    (128, True, 65, 4100, 8192, 4, 4, False, False), (64, True, 64, 4097, 4096, 6, 5, True, True), (256, True, 200, 4865, 8192, 6, 6, True, True),
+    (128, True, 129, 2561, 8192, 7, 7, True, False), (32, True, 20, 1001, 8192, 8, 8, False, False), (256, True, 200, 4865, 8192, 4, 4, True, True),
 ]
 
 
-@pytest.mark.parametrize("split", [0, 1])
-@pytest.mark.parametrize("case", INT_CASES, ids=lambda c: "M{}N{}K{}a{}w{}{}{}".format(*c[:5], "s" if c[5] else "u", "s" if c[6] else "u"))
-def test_int32(abq, oracle, cuda, case, split, monkeypatch):
-    monkeypatch.setenv("ABQ_TC_SPLIT", str(split))
-    M, N, K, p, q, xs, ws = case
+@pytest.mark.parametrize("case", INT_CASES, ids=lambda c: "bt{}{}-M{}N{}K{}a{}w{}{}{}".format(c[0], "cut" if c[1] else "", *c[2:7], "s" if c[7] else "u",
+                                                                                           "s" if c[8] else "u"))
+def test_int32(abq, oracle, cuda, case, monkeypatch):
+    bt, split, M, N, K, p, q, xs, ws = case
+    force(monkeypatch, bt, split)
     rng = np.random.default_rng(M + N + K + q)
     x, w = rand_codes(rng, M, K, p, xs), rand_codes(rng, N, K, q, ws)
     got, st = run_gemm(abq, planes_dev(oracle, x, p), planes_dev(oracle, w, q), M, N, K, x_bits=p, w_bits=q, x_signed=xs, w_signed=ws,
                        route=abq.ROUTE_I8_UMMA)
+    assert plan_of(abq, st) == ("tc_kernel", bt, split)
     want = oracle.gemm_values_blas(x, w)
     assert np.array_equal(got, want), f"{np.count_nonzero(got != want)} of {got.size} differ"
 
 
-@pytest.mark.parametrize("bt", [16, 32, 64, 128])
-@pytest.mark.parametrize("M,N,K,q,group,xs,with_zero", [(16, 200, 1024, 2, 64, True, True), (61, 520, 2944, 4, 128, True, True),
-                                                        (130, 300, 1280, 3, 640, True, True), (40, 256, 1536, 8, 64, False, False),
-                                                        (100, 129, 640, 7, 128, False, True)])
+@pytest.mark.parametrize("M,N,K", [(1, 2048, 4096), (100, 10007, 2944), (256, 4096, 1024), (300, 1001, 2048)])
+def test_int32_as_planned(abq, oracle, cuda, M, N, K):
+    """The planner's own choice of tile and cut."""
+    rng = np.random.default_rng(M)
+    x, w = rand_codes(rng, M, K, 4, True), rand_codes(rng, N, K, 4, False)
+    got, st = run_gemm(abq, planes_dev(oracle, x, 4), planes_dev(oracle, w, 4), M, N, K, x_bits=4, w_bits=4, x_signed=True, w_signed=False,
+                       route=abq.ROUTE_I8_UMMA)
+    assert plan_of(abq, st)[0] == "tc_kernel"
+    assert np.array_equal(got, oracle.gemm_values_blas(x, w))
+
+
+@pytest.mark.parametrize("bt", [16, 32, 64])
+@pytest.mark.parametrize("M,N,K,q,group,xs,with_zero", [(16, 1300, 8192, 2, 64, True, True), (61, 1300, 8192, 4, 128, True, True),
+                                                        (100, 1300, 5120, 3, 640, True, True), (40, 1300, 8192, 8, 64, False, False),
+                                                        (100, 1300, 8192, 7, 128, False, True), (33, 1301, 8320, 5, 64, True, True)])
 def test_scale_groups(abq, oracle, cuda, M, N, K, q, group, xs, with_zero, bt, monkeypatch):
-    """Odd group counts, groups of half a K block and of several, unsigned x unsigned sums above 2^22, K runs cut inside a group."""
-    monkeypatch.setenv("ABQ_TC_BT", str(bt))
+    """Odd group counts, groups of half a K block and of several, unsigned x unsigned sums above 2^22, K cut or not, inside runs of groups."""
     rng = np.random.default_rng(M + K + q)
     x, w = rand_codes(rng, M, K, 8, xs), rand_codes(rng, N, K, q, False)
     G = K // group
     scale = rng.uniform(0.001, 0.02, size=(N, G)).astype(np.float16)
     zero = rng.integers(0, 1 << q, size=(N, G)).astype(np.uint8) if with_zero else None
     tok = rng.uniform(0.001, 0.01, size=M).astype(np.float32)
-    for split in ("0", "1"):
-        monkeypatch.setenv("ABQ_TC_SPLIT", split)
-        got, st = run_gemm(abq, planes_dev(oracle, x, 8), planes_dev(oracle, w, q), M, N, K, x_bits=8, w_bits=q, x_signed=xs, w_signed=False,
-                           out_fp16=True, scale_mode=abq.SCALE_GROUP, group_size=group, w_scale=dev(scale),
-                           w_zero=None if zero is None else dev(zero), x_scale=dev(tok), route=abq.ROUTE_I8_UMMA)
-        check_close(got, oracle.dequant_gemm(x, w, scale, None if zero is None else zero.astype(np.int32), tok, group))
+    ref = oracle.dequant_gemm(x, w, scale, None if zero is None else zero.astype(np.int32), tok, group)
+    xp, wp = planes_dev(oracle, x, 8), planes_dev(oracle, w, q)
+    for split in (False, True):
+        force(monkeypatch, bt, split)
+        got, st = run_gemm(abq, xp, wp, M, N, K, x_bits=8, w_bits=q, x_signed=xs, w_signed=False, out_fp16=True, scale_mode=abq.SCALE_GROUP,
+                           group_size=group, w_scale=dev(scale), w_zero=None if zero is None else dev(zero), x_scale=dev(tok), route=abq.ROUTE_I8_UMMA)
+        assert plan_of(abq, st) == ("tc_kernel", bt, split)
+        check_close(got, ref)
 
 
+@pytest.mark.parametrize("M,K,q,group", [(130, 1280, 3, 640), (129, 1152, 4, 64), (300, 1408, 7, 128)])
+def test_scale_groups_over_expanded_codes(abq, oracle, cuda, M, K, q, group):
+    N = 300
+    rng = np.random.default_rng(M + K + q)
+    x, w = rand_codes(rng, M, K, 8, True), rand_codes(rng, N, K, q, False)
+    scale = rng.uniform(0.001, 0.02, size=(N, K // group)).astype(np.float16)
+    zero = rng.integers(0, 1 << q, size=(N, K // group)).astype(np.uint8)
+    tok = rng.uniform(0.001, 0.01, size=M).astype(np.float32)
+    got, st = run_gemm(abq, planes_dev(oracle, x, 8), planes_dev(oracle, w, q), M, N, K, x_bits=8, w_bits=q, x_signed=True, w_signed=False,
+                       out_fp16=True, scale_mode=abq.SCALE_GROUP, group_size=group, w_scale=dev(scale), w_zero=dev(zero), x_scale=dev(tok))
+    assert plan_of(abq, st) == ("tc_kernel (codes)", 128, False)
+    check_close(got, oracle.dequant_gemm(x, w, scale, zero.astype(np.int32), tok, group))
+
+
+@pytest.mark.parametrize("split", [False, True])
 @pytest.mark.parametrize("q,w_signed", [(1, False), (2, True), (3, False), (3, True), (4, False), (5, True), (7, False), (8, False), (8, True)])
-def test_channel_zero_points(abq, oracle, cuda, q, w_signed):
-    """Zero points subtracted in the codes (up to three bits, unsigned) or times the token's code sum, K runs cut or not; two tiles of
-    tokens, the second one ragged."""
-    M, N, K = 70, 300, 1408
+def test_channel_zero_points(abq, oracle, cuda, q, w_signed, split, monkeypatch):
+    """Zero points subtracted in the codes (two and three bits, unsigned) or times the token's code sum, K cut or not; tiles of 32
+    tokens, the last one ragged."""
+    M, N, K = 70, 700, 8192
+    force(monkeypatch, 32, split)
     rng = np.random.default_rng(q)
     x, w = rand_codes(rng, M, K, 8, True), rand_codes(rng, N, K, q, w_signed)
     scale = rng.uniform(0.001, 0.02, size=N).astype(np.float16)
@@ -64,8 +108,68 @@ def test_channel_zero_points(abq, oracle, cuda, q, w_signed):
     xs = rng.uniform(0.05, 0.2, size=M).astype(np.float32)
     got, st = run_gemm(abq, planes_dev(oracle, x, 8), planes_dev(oracle, w, q), M, N, K, x_bits=8, w_bits=q, x_signed=True, w_signed=w_signed,
                        route=abq.ROUTE_I8_UMMA, out_fp16=True, scale_mode=abq.SCALE_CHANNEL, w_scale=dev(scale), w_zero=dev(zero), x_scale=dev(xs))
+    assert plan_of(abq, st) == ("tc_kernel", 32, split)
     acc = oracle.gemm_values_blas(x, w).astype(np.float64) - zero.astype(np.float64)[None, :] * x.sum(axis=1, dtype=np.int64)[:, None]
     check_close(got, acc * scale.astype(np.float64)[None, :] * xs.astype(np.float64)[:, None])
+
+
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("M,q", [(17, 4), (25, 2), (32, 8)])
+@pytest.mark.parametrize("mode", ["channel", "tensor"])
+def test_residual_by_auto(abq, oracle, cuda, M, q, mode, split, monkeypatch):
+    """AUTO at 17 to 32 rows plans tc_kernel for large matrices, with its residual input: the fp16 add of the result without one."""
+    from abq_llm_b200 import binding as B
+    N, K = 4096, 4096
+    force(monkeypatch, 32, split)
+    rng = np.random.default_rng(M)
+    x, w = rand_codes(rng, M, K, 8, True), rand_codes(rng, N, K, q, False)
+    if mode == "tensor":
+        x = np.fix(x / 64).astype(np.int32)  # sums that fp16 holds
+    kw = dict(scale_mode=abq.SCALE_TENSOR_COMPAT, C=dev(np.array([0.0023], dtype=np.float16)))
+    if mode == "channel":
+        kw = dict(scale_mode=abq.SCALE_CHANNEL, w_scale=dev(rng.uniform(1e-4, 1e-3, size=N).astype(np.float16)),
+                  w_zero=dev(rng.integers(0, 1 << q, size=N, dtype=np.uint8)), x_scale=dev(rng.uniform(0.05, 0.2, size=M).astype(np.float32)))
+    ws = dev(np.zeros(abq.gemm_workspace_bytes(M, N, K, 8, q), dtype=np.uint8))
+    xp, wp = planes_dev(oracle, x, 8), planes_dev(oracle, w, q)
+    res = rng.normal(0, 1, size=(M, N)).astype(np.float16)
+    outs = []
+    for residual in (None, dev(res)):
+        out = dev(np.zeros((M, N), dtype=np.float16))
+        prm = B.make_params(M, N, K, xp, wp, out, x_bits=8, w_bits=q, x_signed=True, w_signed=False, out_dtype=abq.OUT_FP16, workspace=ws,
+                            residual=residual, **kw)
+        st = abq.gemm_init(prm)
+        assert plan_of(abq, st) == ("tc_kernel", 32, split)
+        abq.gemm_exec(st)
+        outs.append(out.cpu().numpy())
+    assert np.isfinite(outs[0].astype(np.float32)).all() and np.abs(outs[0]).max() > 0.1
+    assert np.array_equal(outs[1].view(np.uint16), (outs[0] + res).view(np.uint16))
+
+
+@pytest.mark.parametrize("q", [2, 3, 4])
+@pytest.mark.parametrize("M", [20, 100])
+def test_fp16_activations(abq, oracle, cuda, M, q):
+    """ABQ_FLAG_X_HALF: the codes written in the order of the weights' expansion (its own for two and three bits) give the bits that
+    the quantiser's planes give, and the oracle's result."""
+    from abq_llm_b200 import binding as B
+    N, K, p = 1000, 1152, 8
+    rng = np.random.default_rng(M + q)
+    x = dev(rng.normal(0, 1, size=(M, K)).astype(np.float16))
+    w = rand_codes(rng, N, K, q, False)
+    qs = dev(np.array([20.0], dtype=np.float32))
+    planes = dev(np.zeros((p, M, K // 32), dtype=np.int32))
+    abq.quantize_pack_half(x, qs, planes, M, K, p, 0)
+    wp, ws = planes_dev(oracle, w, q), dev(np.zeros(abq.gemm_workspace_bytes(M, N, K, p, q, abq.ROUTE_I8_UMMA), dtype=np.uint8))
+    outs = []
+    for X, flags in ((planes, 0), (x, abq.FLAG_X_HALF)):
+        out = dev(np.zeros((M, N), dtype=np.int32))
+        prm = B.make_params(M, N, K, X, wp, out, x_bits=p, w_bits=q, x_signed=True, w_signed=False, route=abq.ROUTE_I8_UMMA, flags=flags,
+                            x_quant_scale=qs, workspace=ws)
+        st = abq.gemm_init(prm)
+        assert plan_of(abq, st)[0] == "tc_kernel"
+        abq.gemm_exec(st)
+        outs.append(out.cpu().numpy())
+    assert np.array_equal(outs[0], oracle.gemm_values_blas(oracle.unpack(planes.cpu().numpy().view(np.uint32), True), w))
+    assert np.array_equal(outs[0], outs[1])
 
 
 @pytest.mark.parametrize("M", [24, 100, 200])
