@@ -226,7 +226,13 @@ def gemm(params: GemmParams, stream=None) -> None:
 
 
 STATIC_SCRATCH_BYTES = 16 << 20
-WORKSPACE_COUNTER_BYTES = 256 << 10  # the part of gemm_workspace_bytes() that only plans sharing a workspace need
+WORKSPACE_COUNTER_BYTES = 256 << 10
+
+
+def workspace_sharing_bytes(M: int, N: int, K: int, route: int = ROUTE_AUTO) -> int:
+    """The part of gemm_workspace_bytes() that only plans sharing a workspace need (abq_workspace_sharing_bytes in the header)."""
+    umma = route == ROUTE_I8_UMMA or (route == ROUTE_AUTO and M > 16)
+    return WORKSPACE_COUNTER_BYTES if umma and (M > 128 or N * K < 2 * WORKSPACE_COUNTER_BYTES) else 0
 
 
 def gemm_static_scratch(params: GemmParams, stream=None) -> None:

@@ -61,10 +61,12 @@ abq_status decode_plan(abq_gemm_state *st, bool clear_counters);
 cudaError_t decode_clear_counters(const abq_gemm_state *st, cudaStream_t stream);
 cudaError_t decode_launch(const abq_gemm_state *st, cudaStream_t stream);
 size_t decode_workspace_bytes(int M, int N, int K);
-// split-K scratch shared by both decode kernels: [tile counters][partial slots for kDecodeMaxSlices slices].  The counters have to outlive
-// the launches of every plan that shares the workspace: no plan puts anything else into its first ABQ_WORKSPACE_COUNTER_BYTES, where the
-// workspace has room for that
-void decode_workspace_layout(int M, int N, size_t bytes, size_t *off_partials, size_t *total); // in a workspace of `bytes`
+// Split-K scratch of both decode kernels: tile counters at the start of the workspace, partial slots at its end.  The counters have to
+// outlive the launches of every plan that shares the workspace.  A smaller matrix has fewer slots, so they start behind the counters
+// of a larger one; the tensor-core route leaves the first ABQ_WORKSPACE_COUNTER_BYTES alone.
+size_t decode_counter_bytes(int N);                                    // rounded up to 256
+size_t decode_slots_offset(int N, size_t slot_bytes, size_t bytes);    // in a workspace of `bytes` (0: does not fit)
+size_t decode_slot_bytes(int rows, int N, int slices);                 // `rows` of a launch, 16 features per tile
 
 // ---- gemm_stream.cu (route ABQ_ROUTE_I8_MMA over prepared weights, ABQ_FLAG_WEIGHTS_PREPARED + w_prepared)
 bool stream_supported(const abq_gemm_params &p);
@@ -101,7 +103,7 @@ cudaError_t tc_prepare_x(const abq_gemm_state *st, cudaStream_t stream); // acti
 cudaError_t tc_launch(const abq_gemm_state *st, cudaStream_t stream);
 
 // ---- api.cu helpers
-size_t gemm_scratch_bytes(int M, int N, int K, int route); // abq_gemm_workspace_bytes() without ABQ_WORKSPACE_COUNTER_BYTES
+size_t gemm_scratch_bytes(int M, int N, int K, int route); // abq_gemm_workspace_bytes() without abq_workspace_sharing_bytes()
 // Encodes a tiled TMA descriptor through the driver entry point (no link-time libcuda dependency).
 // dims/strides innermost first; strides in bytes for dimensions 1..rank-1.
 enum TmapSwizzle { TMAP_SWIZZLE_NONE = 0, TMAP_SWIZZLE_32B = 1, TMAP_SWIZZLE_64B = 2, TMAP_SWIZZLE_128B = 3 };

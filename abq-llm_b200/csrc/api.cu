@@ -146,8 +146,7 @@ size_t abq_gemm_workspace_bytes(int M, int N, int K, int x_bits, int w_bits, int
 {
     (void)x_bits;
     (void)w_bits;
-    const size_t need = gemm_scratch_bytes(M, N, K, route);
-    return need ? need + ABQ_WORKSPACE_COUNTER_BYTES : 0;
+    return gemm_scratch_bytes(M, N, K, route) + abq_workspace_sharing_bytes(M, N, K, route);
 }
 
 } // extern "C"

@@ -6,7 +6,7 @@ namespace abq {
 
 struct DecodeLayout {
     int MT, NW, tiles, total_groups, slices, stages_per_slice, ctas_per_slice, split, stages_per_split, ring;
-    size_t smem, off_partials, bytes;
+    size_t smem;
 };
 
 static int device_sms()
@@ -17,25 +17,23 @@ static int device_sms()
     return 148;
 }
 
-// Workspace (only used when K is split over CTAs): [tile counters][partial slots for kDecodeMaxSlices slices].  The slots start behind
-// the room that all plans leave to counters (another plan's may reach further than this one's), in a workspace that has it.
-void decode_workspace_layout(int M, int N, size_t bytes, size_t *off_partials, size_t *total)
+// Workspace (only used when K is split over CTAs)
+size_t decode_counter_bytes(int N) { return ((size_t)((N + 15) / 16) * 4 + 255) & ~(size_t)255; }
+
+size_t decode_slot_bytes(int rows, int N, int slices) { return (size_t)slices * ((N + 15) / 16) * rows * 16 * 4; }
+
+size_t decode_slots_offset(int N, size_t slot_bytes, size_t bytes)
 {
-    const int tiles = (N + 15) / 16;
-    const int rows = M < 16 ? M : 16; // taller problems run as launches of 16 rows, one after the other
-    const size_t slots = (size_t)kDecodeMaxSlices * tiles * rows * 16 * 4;
-    *off_partials = ((size_t)tiles * 4 + 255) & ~(size_t)255;
-    if (*off_partials < ABQ_WORKSPACE_COUNTER_BYTES && bytes >= ABQ_WORKSPACE_COUNTER_BYTES + slots)
-        *off_partials = ABQ_WORKSPACE_COUNTER_BYTES;
-    *total = *off_partials + slots;
+    return bytes < decode_counter_bytes(N) + slot_bytes ? 0 : (bytes - slot_bytes) & ~(size_t)255;
 }
+
+// (taller problems run as launches of 16 rows, one after the other)
+static size_t slot_bytes_of(int M, int N) { return decode_slot_bytes(M < 16 ? M : 16, N, kDecodeMaxSlices); }
 
 size_t decode_workspace_bytes(int M, int N, int K)
 {
     (void)K;
-    size_t a, total;
-    decode_workspace_layout(M, N, 0, &a, &total);
-    return total;
+    return decode_counter_bytes(N) + slot_bytes_of(M, N);
 }
 
 // Launch shape.  K is split over CTAs only as far as needed for the activation records of a slice to fit beside a
@@ -112,7 +110,6 @@ static bool make_layout(const abq_gemm_params &p, DecodeLayout *L)
     L->stages_per_split = (sps + best_split - 1) / best_split;
     L->ring = ring;
     L->smem = fixed + (size_t)sps * 4 * rec + (size_t)NW * ring * stage_bytes;
-    decode_workspace_layout(p.M, p.N, p.workspace_bytes, &L->off_partials, &L->bytes);
     return L->smem <= 227 * 1024;
 }
 
@@ -130,7 +127,7 @@ abq_status decode_plan(abq_gemm_state *st, bool clear_counters)
     DecodeLayout L;
     if (!make_layout(p, &L))
         return ABQ_ERR_UNSUPPORTED;
-    if (L.slices > 1 && (!p.workspace || p.workspace_bytes < L.bytes))
+    if (L.slices > 1 && (!p.workspace || p.workspace_bytes < decode_workspace_bytes(p.M, p.N, p.K)))
         return ABQ_ERR_WORKSPACE;
     if (L.slices > 1 && clear_counters) {
         // K split over CTAs: one arrival counter per tile, zero between launches (every launch leaves them zero).
@@ -174,8 +171,6 @@ cudaError_t decode_launch(const abq_gemm_state *st, cudaStream_t stream)
         return stream_launch(st, stream);
     const abq_gemm_params &p = st->p;
     const int MT = (p.M < 16 ? p.M : 16) <= 8 ? 1 : 2; // as planned: by the rows of a full launch
-    size_t off_partials, total;
-    decode_workspace_layout(p.M, p.N, p.workspace_bytes, &off_partials, &total);
     uint8_t *ws = reinterpret_cast<uint8_t *>(p.workspace);
     const int tiles = (p.N + 15) / 16;
     DecodeArgs a;
@@ -205,8 +200,7 @@ cudaError_t decode_launch(const abq_gemm_state *st, cudaStream_t stream)
     if (a.slices > 1) {
         // the arrival counters are zero here: planning (or the one-shot call) cleared them, every launch leaves them zero
         a.counters = reinterpret_cast<int *>(ws);
-        a.partials = reinterpret_cast<int *>(ws + off_partials);
-
+        a.partials = reinterpret_cast<int *>(ws + decode_slots_offset(p.N, slot_bytes_of(p.M, p.N), p.workspace_bytes));
     }
     a.D = p.D;
     a.w_scale = reinterpret_cast<const __half *>(p.w_scale);

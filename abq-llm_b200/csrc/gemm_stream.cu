@@ -274,10 +274,7 @@ static bool make_plan(const abq_gemm_params &p, StreamPlan *P, size_t *smem_byte
 {
     if (p.M > 16 && env_int("ABQ_STREAM_ROWS32", 0) != 0 && make_plan_rows(p, p.M < 32 ? p.M : 32, P, smem_bytes)) {
         // a K split parks 32-row partial tiles in the workspace, which callers size for 16-row launches: take it only if they fit
-        size_t off_partials, total;
-        decode_workspace_layout(p.M, p.N, p.workspace_bytes, &off_partials, &total);
-        const size_t need = off_partials + (size_t)P->slices * ((p.N + 15) / 16) * 32 * 16 * 4;
-        if (P->slices == 1 || (p.workspace && p.workspace_bytes >= need)) {
+        if (P->slices == 1 || (p.workspace && decode_slots_offset(p.N, decode_slot_bytes(32, p.N, P->slices), p.workspace_bytes) > 0)) {
             P->rows_per_launch = 32;
             return true;
         }
@@ -382,10 +379,10 @@ cudaError_t stream_launch(const abq_gemm_state *st, cudaStream_t stream)
     a.counters = nullptr;
     a.partials = nullptr;
     if (P.slices > 1) {
-        size_t off_partials, total;
-        decode_workspace_layout(p.M, p.N, p.workspace_bytes, &off_partials, &total);
+        const int rows = p.M < P.rows_per_launch ? p.M : P.rows_per_launch;
+        const size_t slots = decode_slot_bytes(rows, p.N, rows > 16 ? P.slices : kDecodeMaxSlices);
         a.counters = reinterpret_cast<int *>(p.workspace);
-        a.partials = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(p.workspace) + off_partials);
+        a.partials = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(p.workspace) + decode_slots_offset(p.N, slots, p.workspace_bytes));
     }
     a.w_scale = reinterpret_cast<const __half *>(p.w_scale);
     a.w_zero = p.w_zero;

@@ -49,7 +49,7 @@ class ABQGEMMWrapper:
              stream=None) -> None:
         if K < 128 or K % 128 != 0:
             raise B.AbqError(1, f"[ABQ][Error] unsupport K = {K}")
-        need = self.workspace_bytes(M, N, K) - B.WORKSPACE_COUNTER_BYTES  # (no plan is kept: nothing shares the workspace)
+        need = self.workspace_bytes(M, N, K) - B.workspace_sharing_bytes(M, N, K)  # (no plan is kept: nothing shares the workspace)
         if abq_gemm_ws_bytes < need:
             raise B.AbqError(3, f"workspace of {abq_gemm_ws_bytes} bytes, {need} needed")
         ws = abq_gemm_workspace

@@ -143,7 +143,7 @@ typedef struct abq_gemm_params {
     const float *x_scale;   /* optional per-token fp32 scale [M], NULL = 1 */
     int route;              /* abq_route */
     int flags;              /* ABQ_FLAG_* */
-    void *workspace;        /* >= abq_gemm_workspace_bytes() (ABQ_WORKSPACE_COUNTER_BYTES less where no other plan shares it), 256-byte aligned */
+    void *workspace;        /* >= abq_gemm_workspace_bytes(), 256-byte aligned */
     size_t workspace_bytes;
     int *status_word;       /* optional device int, set non-zero by a kernel whose bounded wait expired */
     const float *x_quant_scale; /* ABQ_FLAG_X_HALF: device float, the static activation scale */
@@ -172,10 +172,18 @@ typedef struct abq_gemm_state {
     abq_fused_allreduce ar;         /* copy of *p.allreduce (world == 0: none) */
 } abq_gemm_state;
 
-/* Bytes of caller-owned scratch a GEMM of this shape may need (route AUTO: the maximum over routes).  The first
- * ABQ_WORKSPACE_COUNTER_BYTES belong to the arrival counters of plans that split K over CTAs (4 bytes per 16 output features, so
- * up to 1 Mi features); other plans leave them alone, which is what lets plans share a workspace. */
+/* A workspace starts with the arrival counters of plans that split K over CTAs (4 bytes per 16 output features).  The tensor-core
+ * route (I8_UMMA, AUTO above 16 rows) leaves the first ABQ_WORKSPACE_COUNTER_BYTES alone (room for 1 Mi features), which is what lets its
+ * plans share a workspace with the others.  Up to 128 rows they come out of its scratch; otherwise abq_gemm_workspace_bytes() has
+ * abq_workspace_sharing_bytes() in it for them.  A workspace without those is taken all the same, but then must not be shared. */
 #define ABQ_WORKSPACE_COUNTER_BYTES ((size_t)256 << 10)
+static inline size_t abq_workspace_sharing_bytes(int M, int N, int K, int route)
+{
+    const int umma = route == ABQ_ROUTE_I8_UMMA || (route == ABQ_ROUTE_AUTO && M > 16);
+    return umma && (M > 128 || (size_t)N * K < 2 * ABQ_WORKSPACE_COUNTER_BYTES) ? ABQ_WORKSPACE_COUNTER_BYTES : 0;
+}
+
+/* Bytes of caller-owned scratch a GEMM of this shape may need (route AUTO: the maximum over routes). */
 ABQ_API size_t abq_gemm_workspace_bytes(int M, int N, int K, int x_bits, int w_bits, int route);
 
 /*
@@ -321,8 +329,8 @@ ABQ_API abq_status abq_unpack_int8(const void *planes, void *out_i8, int rows, i
  * cudaFree, no allocating library routine), which is what a caller needs that runs inside a stream-ordered forward
  * pass with a workspace it does not size itself (the FasterTransformer linear layers give the GEMM wrapper only
  * x_bits * tokens * K / 8 bytes) and must not synchronise the device.
- *   - Problems whose abq_gemm_workspace_bytes(), less ABQ_WORKSPACE_COUNTER_BYTES, exceeds ABQ_STATIC_SCRATCH_BYTES are
- *     rejected with ABQ_ERR_WORKSPACE; use abq_gemm with a caller-owned workspace for those.
+ *   - Problems whose abq_gemm_workspace_bytes(), less abq_workspace_sharing_bytes(), exceeds ABQ_STATIC_SCRATCH_BYTES
+ *     are rejected with ABQ_ERR_WORKSPACE; use abq_gemm with a caller-owned workspace for those.
  *   - The first call on a device looks the array's address up (cudaGetSymbolAddress, with that device current).
  *     Make that first call outside any stream capture.
  *   - All calls on a device share the one array and it keeps what the last call left in it.  The kernels

@@ -329,7 +329,8 @@ public:
             p.flags |= ABQ_FLAG_WEIGHTS_PREPARED;
             p.route = ABQ_ROUTE_I8_MMA;
         }
-        const size_t need = abq_gemm_workspace_bytes(M, N, K, x_bits_, w_bits_, p.route) - ABQ_WORKSPACE_COUNTER_BYTES; // (one-shot calls)
+        // (no plan is kept here: nothing shares the workspace)
+        const size_t need = abq_gemm_workspace_bytes(M, N, K, x_bits_, w_bits_, p.route) - abq_workspace_sharing_bytes(M, N, K, p.route);
         abq_status s;
         const size_t used = fused ? 0 : plane_bytes; // the fused call leaves the whole workspace to the GEMM
         if (abq_gemm_ws_bytes >= used + need) { // a caller that sized the workspace with room for the scratch

@@ -107,9 +107,9 @@ def test_workspace_sizes(abq):
     assert big > abq.STATIC_SCRATCH_BYTES
 
 
-@pytest.mark.parametrize("M,N,K,route", [(64, 512, 1024, 0), (64, 512, 1024, 3), (16, 512, 11008, 2), (300, 1000, 1152, 0), (64, 16, 128, 3)])
+@pytest.mark.parametrize("M,N,K,route", [(64, 512, 1024, 0), (64, 512, 1024, 3), (16, 512, 11008, 2), (16, 512, 11008, 0), (300, 1000, 1152, 0), (64, 16, 128, 3)])
 def test_a_workspace_without_the_room_for_sharing_is_still_taken(abq, M, N, K, route):
-    """The room for other plans' counters is asked for, not required: without it a plan is made (as far as that goes without a
+    """The tensor-core route asks for room for other plans' counters but does not require it: without it a plan is made (as far as that goes without a
     device: the next step, TMA descriptors or clearing counters, is a CUDA call), with less it is refused."""
     from abq_llm_b200 import binding as B
     p, st = B.GemmParams(), B.GemmState()
@@ -118,7 +118,9 @@ def test_a_workspace_without_the_room_for_sharing_is_still_taken(abq, M, N, K, r
     full = abq.gemm_workspace_bytes(M, N, K, 4, 4, route)
     if torch.cuda.is_available():
         pytest.skip("the addresses are not device memory")
-    for nbytes, status in ((full, 4), (full - abq.WORKSPACE_COUNTER_BYTES, 4), (full - abq.WORKSPACE_COUNTER_BYTES - 512, 3)):
+    least = full - abq.workspace_sharing_bytes(M, N, K, route)
+    assert (least < full) == ((M, N) in ((300, 1000), (64, 16)))
+    for nbytes, status in ((full, 4), (least, 4), (least - 512, 3)):
         p.workspace_bytes = nbytes
         assert abq.lib().abq_gemm_init(ctypes.byref(p), ctypes.byref(st)) == status, nbytes
 

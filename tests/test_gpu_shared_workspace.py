@@ -17,8 +17,9 @@ class Plan:
         self.X = torch.empty((bits, M, K // 32), dtype=torch.int32, device="cuda")
         self.out = torch.full((M, N), -7, dtype=torch.int32, device="cuda")
         self.status = torch.zeros(1, dtype=torch.int32, device="cuda")
-        self.state = abq.gemm_init(B.make_params(M, N, K, self.X, planes, self.out, x_bits=bits, w_bits=bits, x_signed=True, w_signed=False,
-                                                 workspace=ws, status_word=self.status, flags=flags, route=route, **kw))
+        self.params = B.make_params(M, N, K, self.X, planes, self.out, x_bits=bits, w_bits=bits, x_signed=True, w_signed=False,
+                                    workspace=ws, status_word=self.status, flags=flags, route=route, **kw)  # (keeps its tensors)
+        self.state = abq.gemm_init(self.params)
 
     def check(self):
         x = rand_codes(self.rng, self.M, self.K, self.bits, True)
@@ -29,24 +30,35 @@ class Plan:
         assert np.array_equal(self.out.cpu().numpy(), self.oracle.gemm_values_blas(x, self.codes)), f"{self.M} rows"
 
 
-@pytest.mark.parametrize("sizing", ["largest plan", "without the room for sharing"])
-def test_row_counts_in_turn(abq, oracle, cuda, sizing):
+@pytest.mark.parametrize("rows", [(16, 32, 64, 300), (16, 32, 128)])
+def test_row_counts_in_turn(abq, oracle, cuda, rows):
     """Split K (16 rows), the tensor-core kernel over planes (32 rows by AUTO's rule for 16 Mi weights and more; 64) and over expanded codes
-    (300) on one workspace.  In the smaller workspace only the plans over planes still keep clear of the counters."""
+    (300) on one workspace, which the largest asks for.  Up to 128 rows that has no room of its own for the counters."""
     N, K, bits = 1536, 11008, 4
     rng = np.random.default_rng(7)
     w = rand_codes(rng, N, K, bits, False)
     planes = planes_dev(oracle, w, bits)
-    rows = (16, 32, 64, 300) if sizing == "largest plan" else (16, 32, 64)
-    nbytes = abq.gemm_workspace_bytes(rows[-1], N, K, bits, bits)
-    if len(rows) == 3:
-        nbytes -= abq.WORKSPACE_COUNTER_BYTES
-    ws = torch.full((nbytes,), 0xA5, dtype=torch.uint8, device="cuda")
+    ws = torch.full((abq.gemm_workspace_bytes(rows[-1], N, K, bits, bits),), 0xA5, dtype=torch.uint8, device="cuda")
     plans = {M: Plan(abq, oracle, rng, M, N, K, bits, ws, w, planes) for M in rows}
     assert plans[16].state.route == abq.ROUTE_I8_MMA and plans[16].state.cluster > 1, "meant to split K"
     assert plans[32].state.route == abq.ROUTE_I8_UMMA
     for M in [r for m in rows[1:] for r in (16, m)] + [16]:
         plans[M].check()
+
+
+@pytest.mark.parametrize("small", [3072, 4000])
+def test_matrices_of_different_sizes_at_decode_sizes(abq, oracle, cuda, small):
+    """Two split plans in the workspace that the larger one asks for: the smaller one's partial tiles lie behind the larger one's counters."""
+    K, bits = 11008, 4
+    rng = np.random.default_rng(small)
+    ws = torch.full((abq.gemm_workspace_bytes(5, 4096, K, bits, bits),), 0xA5, dtype=torch.uint8, device="cuda")
+    plans = []
+    for N in (4096, small):
+        w = rand_codes(rng, N, K, bits, False)
+        plans.append(Plan(abq, oracle, rng, 5, N, K, bits, ws, w, planes_dev(oracle, w, bits)))
+    assert all(p.state.cluster > 1 for p in plans), "meant to split K"
+    for i in (0, 1, 0, 1):
+        plans[i].check()
 
 
 def test_matrices_of_different_sizes(abq, oracle, cuda):
