@@ -211,7 +211,9 @@ class AbqLinear:
             N, K = self.out_features, self.in_features
             if 16 < M <= 32 and fused is None and (self.w_bits < 8 or K >= 4096 or K <= 1024 or N * K >= 16 << 20):
                 st = self.abq.gemm_init(probe)
-                if st.route != self.abq.ROUTE_I8_UMMA:
+                # (up to 4 bits two launches on the planes beat two on the copy where they beat the one launch: 2048 x 2048 W4
+                # at 17 rows 9.6 us, 10.5 on the copy, 10.4 in one launch)
+                if st.route != self.abq.ROUTE_I8_UMMA and (self.group or self.w_bits > 4 or N * K < 4 << 20):
                     st = None
             if nbytes and st is None:
                 if self.prepared is None:
