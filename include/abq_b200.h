@@ -63,14 +63,18 @@ typedef enum abq_scale_mode {
 } abq_scale_mode;
 
 typedef enum abq_route {
-    ABQ_ROUTE_AUTO = 0,     /* M <= 32 (16 with prepared weights): I8_MMA; otherwise I8_UMMA (per-group scales it cannot fold: I8_MMA) */
+    /* M <= 16: I8_MMA.  17..32: I8_UMMA with ABQ_FLAG_WEIGHTS_PREPARED, and without scale groups for matrices of 4 Mi weights and
+     * more where one launch of it measured faster (and the workspace holds its scratch), otherwise I8_MMA.  Above: I8_UMMA (per-group
+     * scales it cannot fold: I8_MMA). */
+    ABQ_ROUTE_AUTO = 0,
     ABQ_ROUTE_B1_MMA = 1,   /* legacy mma.sync b1 AND+POPC over stacked planes (route A) */
     ABQ_ROUTE_I8_MMA = 2,   /* planes recombined in registers, mma.sync s8/u8, TMA-fed, split-K (decode); M > 16 runs 16 rows per launch */
     ABQ_ROUTE_I8_UMMA = 3   /* planes recombined to int8 tiles, tcgen05.mma kind::i8 in TMEM (route B) */
 } abq_route;
 
 enum {
-    /* Launch with programmatic dependent launch so that consecutive GEMMs overlap.  The decode kernels then request
+    /* Launch with programmatic dependent launch so that consecutive GEMMs overlap.  The kernels that read W as planes or from
+     * w_prepared (all of route I8_MMA; on route I8_UMMA the one for few or ragged rows) then request
      * their first weights BEFORE waiting for the kernel launched ahead of them on the stream: W (or w_prepared) must
      * be complete before that kernel starts -- do not launch a PDL GEMM directly behind the kernel that writes its
      * weights (abq_pack_int32, abq_gemm_prepare_weights, an upload); X, scales and D are read / written after the wait. */
@@ -135,8 +139,8 @@ typedef struct abq_gemm_params {
     int x_signed, w_signed; /* the reference has one SIGNED flag for both (common/base.h QuantType) */
     int out_dtype;          /* abq_out_dtype */
     int scale_mode;         /* abq_scale_mode */
-    int group_size;         /* ABQ_SCALE_GROUP: multiple of 128 dividing K */
-    const void *w_scale;    /* fp16 [N] (CHANNEL) or [N][K/group_size] (GROUP) */
+    int group_size;         /* ABQ_SCALE_GROUP: multiple of 128, or 64, dividing K (some routes take more) */
+    const void *w_scale;    /* fp16 [N] (CHANNEL) or [N][K/group_size] (GROUP), at any fp16 address */
     const uint8_t *w_zero;  /* optional zero points, same shape as w_scale, NULL = 0; each must lie in the code range,
                                0 .. 2^w_bits - 1: the kernels' exactness bounds (int8 operands, the 2^22 bound of the
                                integer-to-float step) assume it and nothing checks device data */
@@ -150,7 +154,8 @@ typedef struct abq_gemm_params {
     void *w_prepared;           /* ABQ_FLAG_WEIGHTS_PREPARED on route I8_MMA: the re-ordered weights, 16-byte aligned */
     const abq_fused_allreduce *allreduce; /* optional (host pointer, copied by abq_gemm_init): sum D over the ranks inside the
                                              GEMM; plans that cannot do it answer ABQ_ERR_UNSUPPORTED */
-    const void *residual;   /* optional fp16 [M][N] (fp16 output; route I8_MMA, or AUTO up to 32 rows; other plans answer ABQ_ERR_UNSUPPORTED):
+    const void *residual;   /* optional fp16 [M][N] (fp16 output; route I8_MMA, or AUTO up to 32 rows -- 16 with ABQ_FLAG_WEIGHTS_PREPARED;
+                               other plans answer ABQ_ERR_UNSUPPORTED):
                                D = half(result) + residual, the fp16 add a separate residual kernel would do after the GEMM
                                (after the sum over the ranks when `allreduce` is set); may alias neither X nor D */
 } abq_gemm_params;
